@@ -119,6 +119,8 @@ struct ppf_plan {
     long xinv_nblk = 0;
     double* ckpt = nullptr;      // Thomas checkpoints of the z solve
     long ckpt_doubles = 0;
+    double* ztab = nullptr;      // tables of the z solve (ZPrep), or null
+    long ztab_len = 0;           // their doubles (0: the z solve takes none)
     float* U = nullptr;          // FP32 first iterate of a refining mixed solve (ghosted layout)
     bool own_work = true;        // A, B, ckpt, partials, U belong to the plan (not to a batch)
     // auxiliary stream of the FP64 low-|k| z solves of the mixed and FP32 paths
@@ -197,7 +199,7 @@ void free_plan(ppf_plan* p)
     if (p->ev_fork) cudaEventDestroy(p->ev_fork);
     if (p->ev_join) cudaEventDestroy(p->ev_join);
     if (p->own_work) {
-        void* work[] = { p->A, p->B, p->partials, p->ckpt, p->U };
+        void* work[] = { p->A, p->B, p->partials, p->ckpt, p->U, p->ztab };
         for (void* q : work)
             if (q) cudaFree(q);
     }
@@ -226,6 +228,39 @@ int validate(const ppf_desc* d)
 }
 
 long round_up(long v, long m) { return (v + m - 1) / m * m; }
+
+// rows of systems the z tables hold (equal eigenvalues stored once)
+int ztab_rows(const ppf_plan* p) { return p->ykind == Y_C2C ? p->my / 2 + 1 : p->my; }
+
+// Doubles of the z tables, 0 where the solve is faster without them.  The
+// tables pay while the chains, not the bytes, bound the z solve.  Measured, a
+// whole solve without -> with tables (spectrum in MB): FP64 with equal
+// eigenvalues shared (a table of a quarter of the spectrum) 128^3 (21) 125 ->
+// 99 us, 256^3 (151) 424 -> 407, 384^3 (491) 1727 -> 1651, 512 x 512 x 128
+// (571) 697 = 697, 512^3 (2282) 2563 -> 2934; others 128 x 128 x 256 (34) 215
+// -> 182, 256^3 real (134) 533 -> 538; cyclic (two tables) 96 x 96 x 200 (29)
+// 244 -> 174, 256 x 256 x 513 (303) 987 -> 1025.  Mixed, one sweep: 256^3 (75)
+// 672 -> 647, 384 x 384 x 192 (123) 1284 -> 1295; real data (an entry is
+// three times its value) 128 x 128 x 256 (17) 377 -> 367, 256^3 (67) 742 -> 764.
+// Mixed solves of tall columns on few cells have no transform long enough to
+// hide the table's chains (128 x 128 x 200 262 -> 274 us, 160^3 348 -> 346,
+// 192^3 529 -> 500), unless the plane is too small to fill the chip (48 x 48
+// x 512 550 -> 297).  The problems of a batch hide their chains behind one
+// another and would pay the tables' bytes: 64 FP64 problems 8.14 -> 8.70 ms.
+long plan_ztab(const ppf_plan* p)
+{
+    const bool f32 = p->elem == 4;
+    if (p->batch_member || (f32 && p->g.pz)) return 0;
+    const long field = p->b_pitch * (long)p->my * p->g.nz * (long)(p->cplx ? 2 : 1) * (long)p->elem;
+    const bool pair = ztab_rows(p) < p->my;
+    long mb = 96;
+    if (!f32 && pair && !p->g.pz) mb = 512;
+    if (f32 && !p->cplx) mb = 32;
+    const long cells = (long)p->g.nx * p->g.ny * p->g.nz;
+    if (f32 && p->g.nz > 160 && cells < 5000000 && p->b_pitch * (long)p->my > 4096) return 0;
+    if (field > (mb << 20)) return 0;
+    return ztab_doubles(p->g.nz, p->b_pitch * (long)ztab_rows(p), p->g.pz, f32);
+}
 
 int plan_init(ppf_plan* p, const ppf_desc* d)
 {
@@ -297,6 +332,7 @@ int plan_init(ppf_plan* p, const ppf_desc* d)
     PPF_CK(cudaMemset(p->scal, 0, sizeof(double) * 8));
     PPF_CK(cudaMemset(p->flags, 0, sizeof(int) * 4));
     p->ckpt_doubles = tdma_z_ckpt_doubles(nz, p->b_pitch * (long)p->my, p->g.pz, p->elem == 4);
+    p->ztab_len = plan_ztab(p);
     if (p->elem == 4) {
         PPF_CK(cudaStreamCreateWithFlags(&p->aux, cudaStreamNonBlocking));
         PPF_CK(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
@@ -322,7 +358,7 @@ size_t u_bytes(const ppf_plan* p)
     return sizeof(float) * (size_t)(p->g.nx + 2) * (p->g.ny + 2) * (p->g.nz + 2);
 }
 
-// the plan's own work memory: spectral buffers, Thomas checkpoints,
+// the plan's own work memory: spectral buffers, Thomas checkpoints or z tables,
 // partials, the FP32 first iterate
 int plan_alloc_work(ppf_plan* p)
 {
@@ -332,7 +368,13 @@ int plan_alloc_work(ppf_plan* p)
         return fail(PPF_ERR_NOMEM, "cannot allocate %.1f MB of spectral work memory",
                     (p->a_bytes + p->b_bytes) / 1048576.0);
     }
-    PPF_CK(cudaMalloc(&p->ckpt, sizeof(double) * p->ckpt_doubles));
+    // the z tables take the place of the checkpoints; without memory for
+    // them the z solve does without
+    if (p->ztab_len && cudaMalloc(&p->ztab, sizeof(double) * p->ztab_len) != cudaSuccess) {
+        cudaGetLastError();
+        p->ztab = nullptr;
+    }
+    if (!p->ztab) PPF_CK(cudaMalloc(&p->ckpt, sizeof(double) * p->ckpt_doubles));
     const long np = partials_doubles(p);
     if (np > 0) {
         p->xinv_nblk = np / 3;
@@ -352,7 +394,7 @@ int plan_alloc_work(ppf_plan* p)
 // residual and the accumulate read it (U_ACC: from p->U).
 template <typename T>
 int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulate, const int* skip,
-             cudaStream_t st, int uk = U_P)
+             cudaStream_t st, int uk = U_P, const double* dx3 = nullptr, const double* dmx3 = nullptr)
 {
     const cx<T>* tw = reinterpret_cast<const cx<T>*>(p->tw);
     const cx<T>* txh = tw + p->tw_off[0];
@@ -377,10 +419,13 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
     z.dzmin2 = p->scal;
     z.dc_shift = p->scal + 4;
     z.cyclic = p->g.pz;
+    z.ypair = p->ykind == Y_C2C;
     z.shared_gpu = p->batch_member ? 1 : 0;
+    z.tab = p->ztab;
+    z.tplane = p->b_pitch * (long)ztab_rows(p);
     z.ckpt = p->ckpt;
-    z.ckpt_f = (sizeof(T) == 4) ? tdma_z_ckpt_f32(p->ckpt, z.nz, z.plane, z.cyclic) : nullptr;
-    if (sizeof(T) == 4 && !z.cyclic) {
+    z.ckpt_f = (sizeof(T) == 4 && !z.tab) ? tdma_z_ckpt_f32(p->ckpt, z.nz, z.plane, z.cyclic) : nullptr;
+    if (sizeof(T) == 4 && !z.cyclic && !z.tab) {
         // the FP64 low-|k| systems: their list, and the table of their
         // coefficient sweeps in the FP64 checkpoint region (unused here)
         z.lowk_count = p->flags + 3;
@@ -389,15 +434,24 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
         z.lowk_cap = tdma_z_ckpt_doubles(z.nz, z.plane, z.cyclic, false);
         z.lowk_build = !resid;
     }
-    cudaError_t e;
+    ZPrep zp{};
+    if (!resid) {
+        // the solve's first launch prepares its z solve in extra blocks
+        zp.dx3 = dx3; zp.dmx3 = dmx3; zp.nz = p->g.nz;
+        zp.am = p->am; zp.ap = p->ap; zp.scal = p->scal; zp.flags = p->flags;
+        zp.lamx = p->lamx; zp.lamy = p->lamy; zp.mx = p->mx; zp.rows = ztab_rows(p); zp.pitch = p->b_pitch;
+        zp.tab = p->ztab; zp.tplane = z.tplane; zp.lowk = z.lowk;
+        zp.f32 = sizeof(T) == 4; zp.cyclic = p->g.pz;
+    }
+    cudaError_t e = launch_xfwd<T>(p->xdct, f, resid ? &rs : nullptr, p->g, p->A, p->a_pitch, p->sx, txh, txn, txd,
+                                   skip, st, resid ? nullptr : &zp);
+    if (e != cudaSuccess) return cuda_fail(e, "x forward");
     if (!resid && z.lowk_list) {
         // the FP64 low-|k| set of this solve (flags[3], zeroed with the
         // flags, counts it); the z solve of every pass uses it
         e = launch_lowk_list(z, st);
         if (e != cudaSuccess) return cuda_fail(e, "low-|k| list");
     }
-    e = launch_xfwd<T>(p->xdct, f, resid ? &rs : nullptr, p->g, p->A, p->a_pitch, p->sx, txh, txn, txd, skip, st);
-    if (e != cudaSuccess) return cuda_fail(e, "x forward");
     mark(p, 1, st);
     // complex views of A and B for the y pass
     const long a_cp = p->xdct ? p->a_pitch / 2 : p->a_pitch;
@@ -434,19 +488,15 @@ int solve_impl(ppf_plan* p, const double* f, double* P, const double* dmx1, cons
     PPF_CK(cudaGetDevice(&cur));
     if (cur != p->dev) return fail(PPF_ERR_STATE, "plan was created on device %d, current device is %d", p->dev, cur);
     mark(p, -1, st);
-    PPF_CK(cudaMemsetAsync(p->flags, 0, sizeof(int) * 4, st));
-    PPF_CK(cudaMemsetAsync(p->scal + 1, 0, sizeof(double) * 7, st));
-    cudaError_t e = launch_zcoef(dx3, dmx3, p->g.nz, p->am, p->ap, p->scal, st);
-    if (e != cudaSuccess) return cuda_fail(e, "z coefficients");
-    mark(p, 0, st);
+    cudaError_t e;
     int rc;
     if (p->elem == 8) {
-        rc = run_pass<double>(p, f, P, false, false, nullptr, st);
+        rc = run_pass<double>(p, f, P, false, false, nullptr, st, U_P, dx3, dmx3);
     } else {
         // a refining mixed solve keeps its first iterate (FP32 values) in U;
         // the first sweep reads it from there and writes P
         const bool u32 = p->d.precision == PPF_MIXED && p->d.max_sweeps > 0 && p->U;
-        rc = run_pass<float>(p, f, P, false, false, nullptr, st, u32 ? U_WRITE : U_P);
+        rc = run_pass<float>(p, f, P, false, false, nullptr, st, u32 ? U_WRITE : U_P, dx3, dmx3);
         if (rc == PPF_OK && p->d.precision == PPF_MIXED) {
             const double ncell = (double)p->g.nx * p->g.ny * p->g.nz;
             e = launch_sweep_gate(p->partials, p->xinv_nblk, ncell, p->scal + 5, p->flags, p->flags + 1,
@@ -631,7 +681,7 @@ int ppf_plan_workspace_bytes(const ppf_plan* plan, long long* bytes)
     if (!plan || !bytes) return fail(PPF_ERR_INVALID, "null argument");
     // spectral buffers, z-solve checkpoints (and low-|k| list), partial sums,
     // the FP32 first iterate of a refining mixed solve
-    *bytes = (long long)(plan->a_bytes + plan->b_bytes + sizeof(double) * plan->ckpt_doubles +
+    *bytes = (long long)(plan->a_bytes + plan->b_bytes + sizeof(double) * (plan->ztab ? plan->ztab_len : plan->ckpt_doubles) +
                          sizeof(double) * partials_doubles(plan) + u_bytes(plan));
     return PPF_OK;
 }
@@ -1068,6 +1118,7 @@ extern "C" int ppf_solve_noalloc(const ppf_desc* desc, const double* f_d, double
     const size_t oFl = off; off = na_align(off + sizeof(int) * 4);
     const size_t oTw = off; off = na_align(off + sizeof(double) * tw_doubles);
     const size_t oCk = off; off = na_align(off + sizeof(double) * tdma_z_ckpt_doubles(nz, p.b_pitch * (long)p.my, p.g.pz, false));
+    const size_t zt = sizeof(double) * (size_t)plan_ztab(&p);   // instead of the checkpoints where it fits
     if (off > (size_t)PPF_NOALLOC_SCRATCH_BYTES)
         return fail(PPF_ERR_UNSUPPORTED,
                     "grid %dx%dx%d needs %zu bytes of work memory; ppf_solve_noalloc holds %zu (use ppf_plan_create)",
@@ -1084,6 +1135,7 @@ extern "C" int ppf_solve_noalloc(const ppf_desc* desc, const double* f_d, double
     p.flags = reinterpret_cast<int*>(b + oFl);
     p.tw = b + oTw;
     p.ckpt = reinterpret_cast<double*>(b + oCk);
+    if (zt && oCk + zt <= (size_t)PPF_NOALLOC_SCRATCH_BYTES) p.ztab = p.ckpt;
 
     cudaStream_t st = (cudaStream_t)stream;
     if (!nd.tables || !same_desc(nd.last, *desc)) {
@@ -1110,7 +1162,6 @@ extern "C" int ppf_solve_noalloc(const ppf_desc* desc, const double* f_d, double
         nd.last = *desc;
         nd.tables = true;
     }
-    PPF_CK(cudaMemsetAsync(p.scal, 0, sizeof(double) * 8, st));
     rc = solve_impl(&p, f_d, p_d, dmx1_d, dmx2_d, dmx3_d, dx3_d, st);
     p.ckpt = nullptr;
     return rc;

@@ -29,7 +29,7 @@ template <typename T>
 cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const Geom& g,
                         void* out, long out_pitch, const FftSched& sch,
                         const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st);
+                        const int* skip_flag, cudaStream_t st, const struct ZPrep* prep = nullptr);
 
 template <typename T>
 cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch,
@@ -78,6 +78,7 @@ struct ZSys {
     double lowk;          // FP32 storage: systems with lam*dz_min^2 < lowk solve in FP64
     const double* dzmin2; // device scalar: min_k dx3_k^2 (written by the z-coefficient kernel)
     double* dc_shift;     // device scalar: z-average of the (0,0) solution (subtracted by the y inverse)
+    int ypair;            // wavenumbers ky and my - ky have equal eigenvalues lamy (complex FFT along y)
     int cyclic;           // periodic z: the reference's cyclic Thomas sequence
     int shared_gpu;       // other solves run beside this one (a batch): no whole-GPU streamed kernel
     double* ckpt;         // Thomas checkpoints, tdma_z_ckpt_doubles(nz, plane, cyclic, fp32) doubles
@@ -88,7 +89,53 @@ struct ZSys {
     double* lowk_tab;     // coefficient table of the first groups (lowk_cap doubles), or null
     long lowk_cap;
     int lowk_build;       // first pass of a solve: fill the table before the z solve
+    // tables of the rhs-independent half of the sweep (ZPrep), or null
+    const double* tab;
+    long tplane;
 };
+
+// Preparation of the z solve, done by the first blocks of a solve's first
+// x-forward launch beside its tiles (zprep in ppf_misc_dev.cuh): the level
+// coefficients, min dz^2, the solve's flags and scalars zeroed and, with
+// `tab`, the half of every z sweep that does not depend on the right-hand
+// side.  Table row k of system i is tab[k * tplane + i]: r_k = 1 / (b_k -
+// a_k c'_{k-1}) below the first row, c'_0 in row 0.  Systems are (kx, ky)
+// rows of `pitch` entries, `rows` of them: with a complex FFT along y only ky
+// <= ny/2, the rest have the same eigenvalues.  Cyclic: r_k of rows 1 ..
+// nz-1 and, nz * tplane further, the back-substituted e_k of the cyclic
+// sequence.  FP32 spectra (f32): r_k of the systems below the low-|k|
+// threshold; the others' FP32 r_k are at (float*)(tab + nz * tplane).
+struct ZPrep {
+    const double* dx3;
+    const double* dmx3;
+    int nz;
+    double* am;
+    double* ap;
+    double* scal;         // [0] min dz^2; [1..7] zeroed
+    int* flags;           // [0..3] zeroed
+    const double* lamx;
+    const double* lamy;
+    int mx, rows;
+    long pitch;
+    double* tab;          // or null
+    long tplane;
+    double lowk;
+    int f32, cyclic;
+};
+// blocks of `threads` threads zprep needs, and their dynamic shared memory
+inline unsigned zprep_blocks(const ZPrep& q, int threads)
+{
+    return q.tab ? (unsigned)((q.pitch * q.rows + threads - 1) / threads) : 1u;
+}
+inline size_t zprep_smem(int nz) { return sizeof(double) * (3 * (size_t)nz + 32); }
+// the preparation in a launch of its own (a solve without tables)
+cudaError_t launch_zprep(const ZPrep& q, cudaStream_t st);
+// doubles of the tables
+inline long ztab_doubles(int nz, long tplane, int cyclic, bool fp32)
+{
+    const long n = tplane * nz;
+    return fp32 ? n + (n + 1) / 2 : (cyclic ? 2 * n : n);
+}
 
 // doubles of checkpoint memory the z solve needs (fp32: FP32 spectral storage)
 long tdma_z_ckpt_doubles(int nz, long plane, int cyclic, bool fp32);
@@ -112,9 +159,6 @@ cudaError_t launch_tdma_z(void* data, const ZSys& z, const int* skip_flag, int* 
 // the low-|k| system list of a mixed or FP32 solve (z.lowk_list), once per
 // solve before its first z solve; a no-op where the list is not used
 cudaError_t launch_lowk_list(const ZSys& z, cudaStream_t st);
-
-cudaError_t launch_zcoef(const double* dx3, const double* dmx3, int nz, double* am, double* ap,
-                         double* dzmin2, cudaStream_t st);
 
 // ---- ghost cells (ppf_ghost.cu) ----
 // zfaces: z faces to fill (1 lower, 2 upper; 3 for a whole domain, the

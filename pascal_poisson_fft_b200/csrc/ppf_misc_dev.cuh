@@ -120,4 +120,127 @@ __device__ __forceinline__ void zcoef(const double* __restrict__ dx3, const doub
     if (threadIdx.x == 0) *dzmin2 = red[0];
 }
 
+// The preparation blocks of a solve (ZPrep): block `blk` of any number of
+// warps, sm: zprep_smem bytes of shared memory.  The coefficients are formed
+// as in zcoef, the table entries by the reference's Thomas operations in
+// their order (thomas_poisson<Exact>; FP32: k_thomas_fast's).  Bound by the
+// latency of its reciprocal chains (about 0.1 us a row), which the transform
+// tiles running beside it hide.
+static __device__ __noinline__ void zprep(const ZPrep& q, unsigned blk, double* sm)
+{
+    const int nz = q.nz, tid = threadIdx.x, nt = blockDim.x;
+    double* const zl = sm;               // am, ap, -am - ap
+    double* const red = sm + 3 * nz;     // 32
+    double mn = INFINITY;
+    for (int k = tid; k < nz; k += nt) {
+        const int kk = k + 1;
+        const double d = q.dx3[kk], inv = __ddiv_rn(1.0, d);
+        double av = __ddiv_rn(inv, q.dmx3[kk]);
+        double cv = __ddiv_rn(inv, q.dmx3[kk + 1]);
+        if (k == 0) av = 0.0;
+        if (k == nz - 1) cv = 0.0;
+        zl[k] = av;
+        zl[nz + k] = cv;
+        zl[2 * nz + k] = __dsub_rn(-av, cv);
+        if (blk == 0) { q.am[k] = av; q.ap[k] = cv; }
+        mn = fmin(mn, d * d);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if ((tid & 31) == 0) red[tid >> 5] = mn;
+    __syncthreads();
+    for (int w = 0; w < (nt >> 5); ++w) mn = fmin(mn, red[w]);
+    if (blk == 0) {
+        if (tid < 8) q.scal[tid] = tid == 0 ? mn : 0.0;
+        if (tid < 4) q.flags[tid] = 0;
+    }
+    if (!q.tab) return;
+    const long idx = (long)blk * nt + tid;
+    const int kx = (int)(idx % q.pitch), ky = (int)(idx / q.pitch);
+    if (kx >= q.mx || ky >= q.rows) return;
+    const double lx = q.lamx[kx], ly = q.lamy[ky];
+    const bool pin = (kx == 0 && ky == 0);
+    auto diag = [&](int k) { return __dsub_rn(__dsub_rn(zl[2 * nz + k], lx), ly); };
+    // The reciprocal chains below form the next row's diagonal ahead of this
+    // row's reciprocal, whose rare-case branch the scheduler does not move
+    // loads and arithmetic across.
+    if (q.f32 && !((lx + ly) * mn < q.lowk)) {
+        float* tab = reinterpret_cast<float*>(q.tab + (size_t)nz * q.tplane) + idx;
+        const float lam = (float)(lx + ly);
+        float cp = __fdividef((float)zl[nz], (float)zl[2 * nz] - lam);
+        tab[0] = cp;
+#pragma unroll 4
+        for (int k = 1; k < nz; ++k) {
+            const float r = __fdividef(1.0f, ((float)zl[2 * nz + k] - lam) - (float)zl[k] * cp);
+            cp = r * (float)zl[nz + k];
+            tab[(size_t)k * q.tplane] = r;
+        }
+        return;
+    }
+    double* tab = q.tab + idx;
+    if (!q.cyclic) {
+        double cp = pin ? 0.0 : __ddiv_rn(zl[nz], diag(0));
+        tab[0] = cp;
+        double a = zl[1], c = zl[nz + 1], b = diag(1);
+#pragma unroll 2
+        for (int k = 1; k < nz; ++k) {
+            const double p = __dsub_rn(b, __dmul_rn(a, cp)), ck = c;
+            const int kn = min(k + 1, nz - 1);
+            a = zl[kn];
+            c = zl[nz + kn];
+            b = diag(kn);
+            const double r = __drcp_rn(p);
+            cp = __dmul_rn(r, ck);
+            tab += q.tplane;
+            *tab = r;
+        }
+        return;
+    }
+    // rows 1 .. nz-1: r and e' (e_1 = -a_1, e_{nz-1} = -c_{nz-1}, the last
+    // one set after the first), then e back-substituted in place
+    double* tabe = tab + (size_t)nz * q.tplane;
+    const double e_last = -zl[nz + nz - 1];
+    double cp = __ddiv_rn(zl[nz + 1], diag(1));
+    double e = __ddiv_rn(nz == 2 ? e_last : -zl[1], diag(1));
+    tab[q.tplane] = cp;
+    tabe[q.tplane] = e;
+    {
+        double a = zl[min(2, nz - 1)], c = zl[nz + min(2, nz - 1)], b = diag(min(2, nz - 1));
+        double *t = tab + q.tplane, *te = tabe + q.tplane;
+#pragma unroll 2
+        for (int k = 2; k < nz; ++k) {
+            const double p = __dsub_rn(b, __dmul_rn(a, cp)), ck = c;
+            const double ei = __dsub_rn(k == nz - 1 ? e_last : 0.0, __dmul_rn(a, e));
+            const int kn = min(k + 1, nz - 1);
+            a = zl[kn];
+            c = zl[nz + kn];
+            b = diag(kn);
+            const double r = __drcp_rn(p);
+            e = __dmul_rn(r, ei);
+            cp = __dmul_rn(r, ck);
+            t += q.tplane;
+            te += q.tplane;
+            *t = r;
+            *te = e;
+        }
+    }
+    for (int k0 = nz - 2; k0 >= 1; k0 -= 8) {
+        double rv[8], ev[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            const int k = k0 - p;
+            rv[p] = ev[p] = 0.0;
+            if (k >= 1) { rv[p] = tab[(size_t)k * q.tplane]; ev[p] = tabe[(size_t)k * q.tplane]; }
+        }
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            const int k = k0 - p;
+            if (k < 1) break;
+            const double c = (k == 1) ? rv[p] : __dmul_rn(rv[p], zl[nz + k]);   // row 1 holds c' itself
+            e = __dsub_rn(ev[p], __dmul_rn(c, e));
+            tabe[(size_t)k * q.tplane] = e;
+        }
+    }
+}
+
 }  // namespace ppf

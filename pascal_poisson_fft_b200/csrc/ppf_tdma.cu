@@ -37,6 +37,7 @@
 #include "ppf_tma.cuh"
 
 #include <math.h>
+#include <algorithm>
 #include <mutex>
 
 namespace ppf {
@@ -1108,9 +1109,331 @@ __global__ void __launch_bounds__(32) k_thomas_lowk(void* __restrict__ data_, ZS
     }
 }
 
+// z solve from the tables of the preparation blocks (ZPrep): with r_k and
+// c'_0 known, the sweeps are multiply-subtract chains without a reciprocal
+// or a branch, d'_k = r_k (d_k - a_k d'_{k-1}), c'_k = r_k c_k, x_k = d'_k -
+// c'_k x_{k+1}: thomas_poisson's operations in the same order (the same bits
+// in FP64).  One lane per real column: the real and the imaginary part of a
+// system are two lanes, so small grids, whose z solve is bound by the chains
+// and not by the field's bytes, have twice the warps at half the work each.
+// KEEP: d' of every row stays in shared memory; else (columns too tall, or
+// too many blocks for the chip at once) it is checkpointed every C rows
+// and recomputed in the substitution.  The rows and table entries of the
+// next chunk load while the current one is swept.  z stage, FP64, with its
+// timing events: 64^3 29 -> 13 us, 128^3 52 -> 19, 256 x 256 x 128 62 -> 47,
+// 384^3 386 -> 286 (k_thomas_exact runs the reciprocal chain twice); cyclic
+// 160 x 128 x 96 66 -> 25; mixed, one sweep, 128^3 67 -> 41, 256^3 165 -> 133.
+constexpr int TAB_TPB = 32;
+constexpr int TAB_C = 16;
+
+// The finite check of a value about to be stored, as exponent bits
+__device__ __forceinline__ unsigned exp_bits(double v) { return (unsigned)__double2hiint(v) & 0x7ff00000u; }
+__device__ __forceinline__ unsigned exp_bits(float v) { return (unsigned)__float_as_int(v) & 0x7f800000u; }
+template <typename CT> constexpr unsigned exp_all = sizeof(CT) == 8 ? 0x7ff00000u : 0x7f800000u;
+
+// One column.  A: arithmetic policy; T: stored field (base, byte offset vo of
+// row 0, vs bytes between rows); R: table entries (likewise); sm: this lane's
+// shared column (TAB_TPB apart): d' per row (KEEP) or per chunk.  32-bit
+// byte offsets and whole chunks without row tests keep the instructions a
+// row low: with a warp or two per scheduler they, not the chain, are the
+// time.  Returns the sum of the scaled column, top row first (of the pinned
+// system only); dtop, xbot: d' of the top row, x of the first; bad: a value
+// is not finite.
+template <bool KEEP, typename A, typename T, typename R>
+__device__ __forceinline__ double tab_sweep(int nz, char* base, unsigned vo, unsigned vs, const char* tbase,
+                                            unsigned to, unsigned ts, const typename A::T* a_,
+                                            const typename A::T* c_, typename A::T* sm, bool pin, typename A::T b0,
+                                            double scale_, typename A::T& dtop, typename A::T& xbot, bool& bad)
+{
+    using CT = typename A::T;
+    constexpr int C = TAB_C;
+    const int nch = (nz + C - 1) / C;
+    const int tail = nz - (nch - 1) * C;   // rows of the top chunk
+    CT va[C], ra[C], vb[C], rb[C];
+    auto load = [&](int ch, CT(&v)[C], CT(&r)[C], bool rows) {
+        const unsigned v0 = vo + (unsigned)(ch * C) * vs, t0 = to + (unsigned)(ch * C) * ts;
+        if (ch < nch - 1 || tail == C) {
+#pragma unroll
+            for (int q = 0; q < C; ++q) {
+                if (rows) v[q] = (CT) * reinterpret_cast<const T*>(base + (size_t)(v0 + q * vs));
+                r[q] = (CT) * reinterpret_cast<const R*>(tbase + (size_t)(t0 + q * ts));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < C; ++q) {
+                if (q < tail) {
+                    if (rows) v[q] = (CT) * reinterpret_cast<const T*>(base + (size_t)(v0 + q * vs));
+                    r[q] = (CT) * reinterpret_cast<const R*>(tbase + (size_t)(t0 + q * ts));
+                }
+            }
+        }
+    };
+    // d' of the rows of chunk ch in v
+    auto elim = [&](int ch, CT(&v)[C], const CT(&r)[C], CT& d) {
+        const CT* al = a_ + ch * C;
+        if (ch == 0) d = A::div(pin ? (CT)0 : v[0], b0);
+        else d = A::mul(r[0], A::sub(v[0], A::mul(al[0], d)));
+        v[0] = d;
+        if (ch < nch - 1 || tail == C) {
+#pragma unroll
+            for (int q = 1; q < C; ++q) v[q] = d = A::mul(r[q], A::sub(v[q], A::mul(al[q], d)));
+        } else {
+#pragma unroll
+            for (int q = 1; q < C; ++q)
+                if (q < tail) v[q] = d = A::mul(r[q], A::sub(v[q], A::mul(al[q], d)));
+        }
+    };
+    CT d = (CT)0;
+    auto fwd = [&](int ch, CT(&v)[C], CT(&r)[C], CT(&v2)[C], CT(&r2)[C]) {
+        if (ch + 1 < nch) load(ch + 1, v2, r2, true);
+        elim(ch, v, r, d);
+        if constexpr (KEEP) {
+            // the shared column holds whole chunks
+            CT* k = sm + ch * C * TAB_TPB;
+#pragma unroll
+            for (int q = 0; q < C; ++q) k[q * TAB_TPB] = v[q];
+        } else {
+            sm[ch * TAB_TPB] = d;
+        }
+    };
+    load(0, va, ra, true);
+    for (int ch = 0; ch < nch; ch += 2) {
+        fwd(ch, va, ra, vb, rb);
+        if (ch + 1 < nch) fwd(ch + 1, vb, rb, va, ra);
+    }
+    dtop = d;
+    CT x = (CT)0;
+    double zsum = 0.0;
+    unsigned top = 0;
+    const CT scale = (CT)scale_;
+    auto bwd = [&](int ch, CT(&v)[C], CT(&r)[C], CT(&v2)[C], CT(&r2)[C]) {
+        if (ch > 0) load(ch - 1, v2, r2, !KEEP);
+        if constexpr (KEEP) {
+            const CT* k = sm + ch * C * TAB_TPB;
+#pragma unroll
+            for (int q = 0; q < C; ++q) v[q] = k[q * TAB_TPB];
+        } else {
+            CT pd = ch > 0 ? sm[(ch - 1) * TAB_TPB] : (CT)0;
+            elim(ch, v, r, pd);
+        }
+        const CT* cl = c_ + ch * C;
+        const unsigned v0 = vo + (unsigned)(ch * C) * vs;
+        // the first row's entry is c' itself
+        r[0] = ch == 0 ? r[0] : A::mul(r[0], cl[0]);
+        auto put = [&](int q) {
+            const CT o = x * scale;
+            v[q] = o;
+            top = max(top, exp_bits(o));
+            *reinterpret_cast<T*>(base + (size_t)(v0 + q * vs)) = (T)o;
+        };
+        if (ch < nch - 1) {
+#pragma unroll
+            for (int q = C - 1; q >= 0; --q) {
+                const CT c = q == 0 ? r[0] : A::mul(r[q], cl[q]);
+                x = A::sub(v[q], A::mul(c, x));
+                put(q);
+            }
+        } else {
+#pragma unroll
+            for (int q = C - 1; q >= 0; --q) {
+                if (q < tail) {
+                    const CT c = q == 0 ? r[0] : A::mul(r[q], cl[q]);
+                    x = (q == tail - 1) ? v[q] : A::sub(v[q], A::mul(c, x));
+                    put(q);
+                }
+            }
+        }
+        if (pin) {
+#pragma unroll
+            for (int q = C - 1; q >= 0; --q)
+                if (ch < nch - 1 || q < tail) zsum += (double)v[q];
+        }
+    };
+    load(nch - 1, va, ra, !KEEP);
+    for (int ch = nch - 1; ch >= 0; ch -= 2) {
+        bwd(ch, va, ra, vb, rb);
+        if (ch > 0) bwd(ch - 1, vb, rb, va, ra);
+    }
+    xbot = x;
+    bad = top >= exp_all<CT>;
+    return zsum;
+}
+
+// rows of the shared column: whole chunks of d' (KEEP) or one per chunk
+__host__ __device__ inline size_t tab_rows(int nz, bool keep)
+{
+    const size_t nch = (size_t)(nz + TAB_C - 1) / TAB_C;
+    return keep ? nch * TAB_C : nch;
+}
+
+template <typename T, bool KEEP>
+size_t tab_smem(int nz)
+{
+    return sizeof(double) * (2 * (size_t)nz + tab_rows(nz, KEEP) * TAB_TPB) +
+           (sizeof(T) == 4 ? 2 * sizeof(float) * (size_t)nz : 0);
+}
+
+template <typename T, bool CPLX, bool KEEP>
+__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
+                                                        int* __restrict__ err)
+{
+    if (skip && *skip) return;
+    constexpr int SH = CPLX ? 1 : 0;
+    extern __shared__ double tab_raw[];
+    const int nz = z.nz;
+    double* const al = tab_raw;
+    double* const cl = al + nz;
+    double* const sm = cl + nz;
+    float* const af = reinterpret_cast<float*>(sm + tab_rows(nz, KEEP) * TAB_TPB);
+    // FP32 spectra: the first half of the grid takes the FP64 systems of its
+    // columns, the second half the FP32 ones, so no warp runs both sweeps
+    const unsigned nb = sizeof(T) == 4 ? gridDim.x / 2 : gridDim.x;
+    const bool fp32 = sizeof(T) == 4 && blockIdx.x >= nb;
+    const unsigned u = (blockIdx.x - (fp32 ? nb : 0u)) * TAB_TPB + threadIdx.x;
+    const unsigned sys = u >> SH;
+    const int kx = (int)(sys % (unsigned)z.pitch), ky = (int)(sys / (unsigned)z.pitch);
+    const bool in = kx < z.mx && ky < z.my;
+    const double lx = in ? z.lamx[kx] : 0.0, ly = in ? z.lamy[ky] : 0.0;
+    const bool high = sizeof(T) == 4 && in && !((lx + ly) * __ldg(z.dzmin2) < z.lowk);
+    const bool mine = in && high == fp32;
+    if (!__any_sync(0xffffffffu, mine)) return;
+    for (int k = threadIdx.x; k < nz; k += TAB_TPB) {
+        const double a = z.am[k], c = z.ap[k];
+        al[k] = a;
+        cl[k] = c;
+        if constexpr (sizeof(T) == 4) { af[k] = (float)a; af[nz + k] = (float)c; }
+    }
+    __syncwarp();
+    if (!mine) return;
+    const bool pin = (kx == 0 && ky == 0);
+    const int kt = (z.ypair && 2 * ky > z.my) ? z.my - ky : ky;
+    char* const base = reinterpret_cast<char*>(data_);
+    const unsigned vo = u * (unsigned)sizeof(T), vs = (unsigned)(z.plane << SH) * (unsigned)sizeof(T);
+    const unsigned ti = (unsigned)(kt * (int)z.pitch + kx);
+    bool bad = false;
+    if constexpr (sizeof(T) == 4) {
+        if (fp32) {
+            const char* tf = reinterpret_cast<const char*>(z.tab + (size_t)nz * z.tplane);
+            const float b0 = (float)__dsub_rn(-al[0], cl[0]) - (float)(lx + ly);
+            // this lane's column in the front half of the doubles' rows
+            float* smf = reinterpret_cast<float*>(sm) + threadIdx.x;
+            float dt, xb;
+            tab_sweep<KEEP, Fast, T, float>(nz, base, vo, vs, tf, ti * 4u, (unsigned)z.tplane * 4u, af, af + nz, smf,
+                                            false, b0, z.scale, dt, xb, bad);
+            if (bad && err) atomicOr(err, 1);
+            return;
+        }
+    }
+    const double b0 = pin ? 1.0 : __dsub_rn(__dsub_rn(__dsub_rn(-al[0], cl[0]), lx), ly);
+    double dt, xb;
+    const double zsum =
+        tab_sweep<KEEP, Exact, T, double>(nz, base, vo, vs, reinterpret_cast<const char*>(z.tab), ti * 8u,
+                                          (unsigned)z.tplane * 8u, al, cl, sm + threadIdx.x, pin, b0, z.scale, dt, xb,
+                                          bad);
+    if (u == 0 && z.dc_shift) *z.dc_shift = zsum / (double)nz;
+    if (bad && err) atomicOr(err, 1);
+}
+
+// The cyclic FP64 sequence (thomas_poisson_cyc<Exact>) from the tables: rows
+// 1 .. nz-1 are solved for y in place, x_0 follows from their ends and the
+// tabulated e, then x_k = y_k + x_0 e_k.
+template <bool CPLX, bool KEEP>
+__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab_cyc(void* __restrict__ data_, ZSys z,
+                                                            const int* __restrict__ skip, int* __restrict__ err)
+{
+    if (skip && *skip) return;
+    using X = Exact;
+    constexpr int SH = CPLX ? 1 : 0, C = TAB_C;
+    extern __shared__ double tab_raw[];
+    const int nz = z.nz;
+    double* const al = tab_raw;
+    double* const cl = al + nz;
+    double* const sm = cl + nz;
+    for (int k = threadIdx.x; k < nz; k += TAB_TPB) {
+        al[k] = z.am[k];
+        cl[k] = z.ap[k];
+    }
+    __syncthreads();
+    const unsigned u = blockIdx.x * TAB_TPB + threadIdx.x;
+    const unsigned sys = u >> SH;
+    const int kx = (int)(sys % (unsigned)z.pitch), ky = (int)(sys / (unsigned)z.pitch);
+    if (kx >= z.mx || ky >= z.my) return;
+    const double lx = z.lamx[kx], ly = z.lamy[ky];
+    const bool pin = (kx == 0 && ky == 0);
+    const int kt = (z.ypair && 2 * ky > z.my) ? z.my - ky : ky;
+    char* const base = reinterpret_cast<char*>(data_);
+    const unsigned vo = u * 8u, vs = (unsigned)(z.plane << SH) * 8u;
+    const unsigned to = (unsigned)(kt * (int)z.pitch + kx) * 8u, ts = (unsigned)z.tplane * 8u;
+    const char* const tab = reinterpret_cast<const char*>(z.tab);
+    const char* const tabe = reinterpret_cast<const char*>(z.tab + (size_t)nz * z.tplane);
+    auto diag = [&](int k) { return X::sub(X::sub(X::sub(-al[k], cl[k]), lx), ly); };
+    auto at = [&](int k) -> double& { return *reinterpret_cast<double*>(base + (size_t)(vo + (unsigned)k * vs)); };
+    auto e_at = [&](int k) { return *reinterpret_cast<const double*>(tabe + (size_t)(to + (unsigned)k * ts)); };
+    const double v0 = pin ? 0.0 : at(0), etop = e_at(nz - 1), e1 = e_at(1);
+    double dtop, y1;
+    bool bad = false;
+    tab_sweep<KEEP, X, double, double>(nz - 1, base, vo + vs, vs, tab, to + ts, ts, al + 1, cl + 1, sm + threadIdx.x,
+                                       false, diag(1), 1.0, dtop, y1, bad);
+    const double a0 = pin ? 0.0 : al[0], c0 = pin ? 0.0 : cl[0], b0 = pin ? 1.0 : diag(0);
+    const double den = X::add(X::add(b0, X::mul(a0, etop)), X::mul(c0, e1));
+    const double x0 = X::div(X::sub(X::sub(v0, X::mul(a0, dtop)), X::mul(c0, y1)), den);
+    double zsum = 0.0;
+    unsigned top = 0;
+    for (int k1 = nz - 1; k1 >= 1; k1 -= C) {
+        double y[C], e[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+            if (k1 - q >= 1) { y[q] = at(k1 - q); e[q] = e_at(k1 - q); }
+#pragma unroll
+        for (int q = 0; q < C; ++q)
+            if (k1 - q >= 1) {
+                const double o = X::add(y[q], X::mul(x0, e[q])) * z.scale;
+                zsum += o;
+                top = max(top, exp_bits(o));
+                at(k1 - q) = o;
+            }
+    }
+    const double o = x0 * z.scale;
+    zsum += o;
+    top = max(top, exp_bits(o));
+    at(0) = o;
+    bad |= top >= exp_all<double>;
+    if (u == 0 && z.dc_shift) *z.dc_shift = zsum / (double)nz;
+    if (bad && err) atomicOr(err, 1);
+}
+
+template <typename T, bool CPLX>
+cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, cudaStream_t st)
+{
+    const unsigned nb = (unsigned)(((z.plane << (CPLX ? 1 : 0)) + TAB_TPB - 1) / TAB_TPB);
+    const unsigned grid = sizeof(T) == 4 ? 2 * nb : nb;
+    // d' in shared memory where every block is resident at once with it (the
+    // 227 KB of each SM's shared memory, 1 KB a block reserved): 48 x 48 x 512
+    // z 52 -> 43 us; more blocks than that would run in waves
+    int dev = 0, sms = 0;
+    cudaError_t de = cudaGetDevice(&dev);
+    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (de != cudaSuccess) return de;
+    const size_t ks = tab_smem<T, true>(z.nz);
+    const bool keep = ks <= 200 * 1024 && (long)nb <= sms * std::min(32L, (long)(227 * 1024 / (ks + 1024)));
+    auto go = [&](auto kern, size_t smem) {
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
+        kern<<<grid, TAB_TPB, smem, st>>>(data, z, skip, err);
+        return cudaGetLastError();
+    };
+    if constexpr (sizeof(T) == 8)
+        if (z.cyclic)
+            return keep ? go(k_thomas_tab_cyc<CPLX, true>, ks) : go(k_thomas_tab_cyc<CPLX, false>, tab_smem<T, false>(z.nz));
+    return keep ? go(k_thomas_tab<T, CPLX, true>, ks) : go(k_thomas_tab<T, CPLX, false>, tab_smem<T, false>(z.nz));
+}
+
 template <bool CPLX, bool CYC>
 cudaError_t launch_z(double*, const ZSys& z, void* data, const int* skip, int* err, const ZStreams& zs)
 {
+    if (z.tab) return launch_tab<double, CPLX>(z, data, skip, err, zs.st);
     dim3 grid((unsigned)((z.plane + TPB - 1) / TPB));  // pitch * my systems incl. padding columns
     if (CYC) k_thomas_z<double, Exact, CPLX, 0, CYC><<<grid, TPB, 0, zs.st>>>(data, z, skip, err);
     else k_thomas_exact<CPLX, true><<<grid, TPB, 3 * sizeof(double) * z.nz, zs.st>>>(data, z, skip, err);
@@ -1122,6 +1445,7 @@ cudaError_t launch_z(double*, const ZSys& z, void* data, const int* skip, int* e
 template <bool CPLX, bool CYC>
 cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* err, const ZStreams& zs)
 {
+    if (z.tab) return launch_tab<float, CPLX>(z, data, skip, err, zs.st);
     dim3 grid((unsigned)((z.plane + TPB - 1) / TPB));
     cudaStream_t lo = zs.st;
     if (zs.aux) {
@@ -1456,17 +1780,16 @@ cudaError_t launch_tdma_update(const double* a, const double* c, double* d, cons
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(256) k_zcoef(const double* __restrict__ dx3, const double* __restrict__ dmx3,
-                                               int nz, double* __restrict__ am, double* __restrict__ ap,
-                                               double* __restrict__ dzmin2)
+// the z preparation alone (one block: no tables)
+__global__ void __launch_bounds__(256) k_zprep(const __grid_constant__ ZPrep zp)
 {
-    zcoef(dx3, dmx3, nz, am, ap, dzmin2);
+    extern __shared__ __align__(16) unsigned char prep_raw[];
+    zprep(zp, blockIdx.x, reinterpret_cast<double*>(prep_raw));
 }
 
-cudaError_t launch_zcoef(const double* dx3, const double* dmx3, int nz, double* am, double* ap, double* dzmin2,
-                         cudaStream_t st)
+cudaError_t launch_zprep(const ZPrep& zp, cudaStream_t st)
 {
-    k_zcoef<<<1, 256, 0, st>>>(dx3, dmx3, nz, am, ap, dzmin2);
+    k_zprep<<<1, 256, zprep_smem(zp.nz), st>>>(zp);
     return cudaGetLastError();
 }
 

@@ -9,6 +9,7 @@
 // here each is one read and one write of the field.  SH selects the
 // compile-time engine of a common length or the run-time engine.
 #include "ppf_tma.cuh"
+#include "ppf_misc_dev.cuh"
 #include "ppf_x_dev.cuh"
 
 #include <type_traits>
@@ -27,21 +28,36 @@ namespace ppf {
     const double* __restrict__ f, ResidIn rs, Geom g, void* __restrict__ out_, long out_pitch, FftSched sch,    \
         int Wrt, int lgWrt, const cx<T>* __restrict__ tw_half, const cx<T>* __restrict__ tw_n,                \
         const cx<T>* __restrict__ tw_dct, const int* __restrict__ skip
-#define PPF_XFWD_ARGS f, rs, g, out_, out_pitch, sch, Wrt, lgWrt, tw_half, tw_n, tw_dct, skip, (long)blockIdx.x
+#define PPF_XFWD_ARGS(tile) f, rs, g, out_, out_pitch, sch, Wrt, lgWrt, tw_half, tw_n, tw_dct, skip, tile
+
+// The x forward of a solve with z tables: the first nprep blocks prepare the
+// z solve beside the transform tiles.  Its own entry point: the call costs
+// the large transforms registers (512^3 mixed solve +1 % with it in k_xfwd).
+template <typename T, bool DCT, typename SH>
+__global__ void __launch_bounds__(512, (SH::CT && SH::NT <= 256) ? 2 : 0)
+    k_xfwd_prep(PPF_XFWD_PARAMS, const __grid_constant__ ZPrep zp, unsigned nprep)
+{
+    if (blockIdx.x < nprep) {
+        extern __shared__ __align__(16) unsigned char prep_raw[];
+        zprep(zp, blockIdx.x, reinterpret_cast<double*>(prep_raw));
+        return;
+    }
+    xfwd<T, DCT, 0, SH>(PPF_XFWD_ARGS((long)blockIdx.x - nprep));
+}
 
 // the plain periodic transform of 384-point tiles (768-point lines) is bounded
 // to four resident CTAs of 384 threads: 32 registers, five CTAs fit an SM
 template <typename T, bool DCT, int RESID, typename SH>
 __global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 : 0) k_xfwd(PPF_XFWD_PARAMS)
 {
-    xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS);
+    xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
 // FP64 compile-time tiles: five resident CTAs of SH::NT threads per SM
 template <bool DCT, typename SH, typename T = double>
 __global__ void __launch_bounds__(SH::NT, 5) k_xfwd64(PPF_XFWD_PARAMS)
 {
-    xfwd<T, DCT, 0, SH>(PPF_XFWD_ARGS);
+    xfwd<T, DCT, 0, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
 // The x stencil ghosts of a tile's lines (the periodic copy, or the wall
@@ -293,11 +309,17 @@ __global__ void __launch_bounds__(SH::NT, (SH::N <= 128) ? 2 : SH::N == 384 ? 3 
 template <typename T>
 cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const Geom& g, void* out, long out_pitch,
                         const FftSched& sch, const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st)
+                        const int* skip_flag, cudaStream_t st, const ZPrep* prep)
 {
     const int nc = g.nx / 2;
     ResidIn rs{};
     if (resid) rs = *resid;
+    if (resid && prep) return cudaErrorInvalidValue;
+    if (prep && !prep->tab) {
+        const cudaError_t e = launch_zprep(*prep, st);
+        if (e != cudaSuccess) return e;
+        prep = nullptr;
+    }
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
         using SH = decltype(sh);
@@ -306,6 +328,17 @@ cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const G
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
         const size_t smem = (size_t)nc * W * sizeof(cx<T>);
         dim3 grid((unsigned)(((long)g.ny * g.nz + W - 1) / W));
+        if (prep) {
+            auto kern = dct ? k_xfwd_prep<T, true, SH> : k_xfwd_prep<T, false, SH>;
+            const size_t psmem = std::max(smem, zprep_smem(prep->nz));
+            const unsigned nprep = zprep_blocks(*prep, threads);
+            err = set_smem(kern, psmem);
+            if (err != cudaSuccess) return;
+            kern<<<grid.x + nprep, threads, psmem, st>>>(f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n,
+                                                        tw_dct, skip_flag, *prep, nprep);
+            err = cudaGetLastError();
+            return;
+        }
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
             if (err != cudaSuccess) return;
@@ -450,19 +483,17 @@ long xinv_blocks(const Geom& g, const FftSched& sch)
     return blocks;
 }
 
-template long xinv_blocks<double>(const Geom&, const FftSched&);
-template long xinv_blocks<float>(const Geom&, const FftSched&);
-
-#define PPF_INST(T)                                                                                        \
-    template cudaError_t launch_xfwd<T>(bool, const double*, const ResidIn*, const Geom&, void*, long,     \
-                                        const FftSched&, const cx<T>*, const cx<T>*, const cx<T>*,         \
-                                        const int*, cudaStream_t);                                         \
-    template cudaError_t launch_xinv<T>(bool, const void*, long, double*, float*, int, const Geom&, bool,  \
-                                        bool,                                                              \
-                                        double*, const double*, const FftSched&, const cx<T>*,             \
-                                        const cx<T>*, const cx<T>*, const int*, cudaStream_t, long*, int*);
-PPF_INST(double)
-PPF_INST(float)
-#undef PPF_INST
+// one element type and direction per compilation unit (build.py)
+#if PPF_FWD
+template cudaError_t launch_xfwd<PPF_REAL>(bool, const double*, const ResidIn*, const Geom&, void*, long,
+                                           const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*,
+                                           const cx<PPF_REAL>*, const int*, cudaStream_t, const ZPrep*);
+#else
+template long xinv_blocks<PPF_REAL>(const Geom&, const FftSched&);
+template cudaError_t launch_xinv<PPF_REAL>(bool, const void*, long, double*, float*, int, const Geom&, bool, bool,
+                                           double*, const double*, const FftSched&, const cx<PPF_REAL>*,
+                                           const cx<PPF_REAL>*, const cx<PPF_REAL>*, const int*, cudaStream_t, long*,
+                                           int*);
+#endif
 
 }  // namespace ppf

@@ -382,15 +382,15 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
     return err;
 }
 
-#define PPF_INST(T)                                                                                        \
-    template cudaError_t launch_yfwd<T>(int, const cx<T>*, long, cx<T>*, long, int, const Geom&,           \
-                                        const FftSched&, const cx<T>*, const cx<T>*, const int*,           \
-                                        cudaStream_t, int*);                                               \
-    template cudaError_t launch_yinv<T>(int, const cx<T>*, long, cx<T>*, long, int, const Geom&,           \
-                                        const FftSched&, const cx<T>*, const cx<T>*, const double*,        \
-                                        const int*, cudaStream_t, int*);
-PPF_INST(double)
-PPF_INST(float)
-#undef PPF_INST
+// one element type and direction per compilation unit (build.py)
+#if PPF_FWD
+template cudaError_t launch_yfwd<PPF_REAL>(int, const cx<PPF_REAL>*, long, cx<PPF_REAL>*, long, int, const Geom&,
+                                           const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*, const int*,
+                                           cudaStream_t, int*);
+#else
+template cudaError_t launch_yinv<PPF_REAL>(int, const cx<PPF_REAL>*, long, cx<PPF_REAL>*, long, int, const Geom&,
+                                           const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*, const double*,
+                                           const int*, cudaStream_t, int*);
+#endif
 
 }  // namespace ppf
