@@ -58,23 +58,66 @@ void cexp_tab(int count, long double num, long double den, std::vector<double>& 
     }
 }
 
-// Radix schedule of a length-n transform.  order 0: radix 8 first, then 4,
-// 2, 3, 5 (fewest passes); 1: no radix 8; 2: radices 3 and 5 first.
-bool factor(int n, FftSched& s, int order_id = 0)
+// The fewest passes, then the largest smallest radix, of a descending radix
+// sequence of n; false if n has a factor other than 2, 3, 5.
+bool few_passes(int n, int top, size_t elem, std::vector<int>& cur, std::vector<int>& best)
 {
-    static const int orders[3][5] = { { 8, 4, 2, 3, 5 }, { 4, 2, 3, 5, 0 }, { 3, 5, 8, 4, 2 } };
+    if (n == 1) {
+        if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && cur.back() > best.back()))
+            best = cur;
+        return true;
+    }
+    if (!best.empty() && cur.size() + 1 > best.size()) return true;
+    bool any = false;
+    for (int r : { 10, 9, 8, 6, 5, 4, 3, 2 }) {
+        if (r > top || n % r || (elem == 8 && (r == 6 || r > 8))) continue;
+        cur.push_back(r);
+        any |= few_passes(n / r, r, elem, cur, best);
+        cur.pop_back();
+    }
+    return any;
+}
+
+// Radix schedule of a length-n transform of FP64 (elem 8) or FP32 (4) data.
+// order 0: the fewest passes (FP64 of radices 2, 3, 4, 5, 8; FP32 also 6, 9,
+// 10; every pass is one round trip of the tile through shared
+// memory and a barrier: 90 = 10 9, 360 = 10 6 6, 720 = 10 9 8, where radices
+// 2, 3, 4, 5, 8 need 4, 5 and 5); 1: radices 4, 2, 3, 5; 2: radices 3 and 5
+// first, then 8, 4, 2.
+bool factor(int n, FftSched& s, size_t elem, int order_id = 0)
+{
+    static const int orders[3][5] = { { 0, 0, 0, 0, 0 }, { 4, 2, 3, 5, 0 }, { 3, 5, 8, 4, 2 } };
     s = FftSched{};
     s.n = n;
     if (n < 1 || order_id < 0 || order_id > 2) return false;
     int m = n;
-    for (int r : orders[order_id]) {
-        while (r > 0 && m % r == 0 && m > 1) {
-            if (s.npass >= 12) return false;
-            s.radix[s.npass++] = r;
-            m /= r;
+    if (order_id == 0) {
+        std::vector<int> cur, best;
+        if (n > 1) {
+            for (int r : { 2, 3, 5 })
+                while (m % r == 0) m /= r;
+            if (m != 1) return false;
+            few_passes(n, 10, elem, cur, best);
+        }
+        if (best.size() > 12) return false;
+        for (int r : best) s.radix[s.npass++] = r;
+    } else {
+        for (int r : orders[order_id]) {
+            while (r > 0 && m % r == 0 && m > 1) {
+                if (s.npass >= 12) return false;
+                s.radix[s.npass++] = r;
+                m /= r;
+            }
         }
     }
     if (n == 1) { s.radix[0] = 2; s.npass = 0; }
+    s.mg_n = div_magic((unsigned)n);
+    s.mg_np = div_magic((unsigned)(n / 2 + 1));
+    unsigned ns = 1;
+    for (int p = 0; p < s.npass; ++p) {
+        s.mg_ns[p] = div_magic(ns);
+        ns *= (unsigned)s.radix[p];
+    }
     return m == 1;
 }
 
@@ -219,8 +262,8 @@ int validate(const ppf_desc* d)
     if (d->max_sweeps > 8) return fail(PPF_ERR_INVALID, "max_sweeps %d > 8", d->max_sweeps);
     if (d->n3m > 1024) return fail(PPF_ERR_UNSUPPORTED, "n3m %d > 1024", d->n3m);
     FftSched s;
-    if (!factor(d->n1m / 2, s)) return fail(PPF_ERR_UNSUPPORTED, "n1m/2 = %d is not a product of 2, 3, 5", d->n1m / 2);
-    if (!factor(d->n2m, s)) return fail(PPF_ERR_UNSUPPORTED, "n2m = %d is not a product of 2, 3, 5", d->n2m);
+    if (!factor(d->n1m / 2, s, 4)) return fail(PPF_ERR_UNSUPPORTED, "n1m/2 = %d is not a product of 2, 3, 5", d->n1m / 2);
+    if (!factor(d->n2m, s, 4)) return fail(PPF_ERR_UNSUPPORTED, "n2m = %d is not a product of 2, 3, 5", d->n2m);
     const int limx = (d->precision == PPF_FP64) ? 2048 : 1024;
     if (d->n1m > limx || d->n2m > 2048)
         return fail(PPF_ERR_UNSUPPORTED, "n1m %d / n2m %d beyond the transform tile limits", d->n1m, d->n2m);
@@ -277,8 +320,8 @@ int plan_init(ppf_plan* p, const ppf_desc* d)
     p->ydct = !d->pbc2;
     p->elem = (d->precision == PPF_FP64) ? 8 : 4;
     const size_t ce = 2 * p->elem;  // complex element bytes
-    factor(nx / 2, p->sx);
-    factor(ny, p->sy);
+    factor(nx / 2, p->sx, p->elem);
+    factor(ny, p->sy, p->elem);
 
     const int nh = nx / 2 + 1;
     if (!p->xdct) {
@@ -1071,8 +1114,8 @@ extern "C" int ppf_solve_noalloc(const ppf_desc* desc, const double* f_d, double
     p.xdct = !desc->pbc1;
     p.ydct = !desc->pbc2;
     p.elem = 8;
-    factor(nx / 2, p.sx);
-    factor(ny, p.sy);
+    factor(nx / 2, p.sx, 8);
+    factor(ny, p.sy, 8);
     const size_t ce = 16;
     const int nh = nx / 2 + 1;
     if (!p.xdct) {
@@ -1441,17 +1484,17 @@ std::vector<TuneChoice> tune_candidates(int n)
 {
     std::vector<TuneChoice> out;
     TuneChoice base{};
-    factor(n, base.s, 0);
+    factor(n, base.s, sizeof(T), 0);
     out.push_back(base);  // default (compile-time shape where one exists)
     int thr = 0;
     const int w0 = pick_w<T>(n, thr);
     for (int o = 0; o < 3; ++o) {
         TuneChoice c{};
-        if (!factor(n, c.s, o)) continue;
+        if (!factor(n, c.s, sizeof(T), o)) continue;
         bool dup = false;
         for (int q = 0; q < o && !dup; ++q) {
             FftSched t{};
-            factor(n, t, q);
+            factor(n, t, sizeof(T), q);
             dup = (t.npass == c.s.npass) && std::equal(t.radix, t.radix + t.npass, c.s.radix);
         }
         if (dup) continue;

@@ -265,8 +265,8 @@ size_t batch_smem(const BProb* probs, int count)
     for (int i = 0; i < count; ++i) {
         const BProb& p = probs[i];
         const size_t ce = 2 * (size_t)p.elem;
-        m = std::max(m, (size_t)(p.g.nx / 2) * p.wx * ce);
-        m = std::max(m, (size_t)p.g.ny * p.wy * ce);
+        m = std::max(m, (size_t)(p.g.nx / 2) * rt_pitch(p.wx) * ce);
+        m = std::max(m, (size_t)p.g.ny * rt_pitch(p.wy) * ce);
     }
     return m;
 }

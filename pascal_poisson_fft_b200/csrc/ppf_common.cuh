@@ -37,20 +37,9 @@ template <> __device__ __forceinline__ cx<float> ldg(const cx<float>* p)
     return mk(v.x, v.y);
 }
 
-// Shared-memory tile layout: element (n, l) of W interleaved lines, row n
-// holds the W lines' n-th elements.  The low bits of the line index are
-// XOR-swizzled with the row so that column-wise writes (one line, many n)
-// and row-wise accesses are both free of bank conflicts.  G = elements per
-// 128-byte bank row; W is a power of two (rows narrower than a bank row
-// are swizzled over W).
+// Complex elements per 128-byte bank row of shared memory, the width of the
+// tiles' line-index swizzle (sidx_ct)
 template <typename T> struct SwizzleG { static constexpr int value = 128 / (int)sizeof(cx<T>); };
-
-template <typename T>
-__device__ __forceinline__ int sidx(int n, int l, int W)
-{
-    constexpr int G = SwizzleG<T>::value;
-    return n * W + (l ^ (n & (W - 1) & (G - 1)));
-}
 
 // Asynchronous global -> shared copies (cp.async): one element per call,
 // completion tracked per thread by commit groups.
@@ -99,6 +88,14 @@ struct FftSched {
     int radix[12];
     int w;    // lines per tile of the run-time engine (0: default width)
     int rt;   // 1: run-time engine even where a compile-time shape exists
+    // fast_div multipliers of the run-time engine: n, n/2 + 1, and the
+    // product of the radices before each pass
+    unsigned mg_n, mg_np, mg_ns[12];
 };
+
+// e / d of small non-negative integers (e d < 2^32) by one multiplication,
+// m = div_magic(d)
+inline unsigned div_magic(unsigned d) { return d < 2 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
+__device__ __forceinline__ int fast_div(int e, unsigned m) { return m ? (int)__umulhi((unsigned)e, m) : e; }
 
 }  // namespace ppf

@@ -326,7 +326,7 @@ cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const G
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
-        const size_t smem = (size_t)nc * W * sizeof(cx<T>);
+        const size_t smem = tile_elems<SH>(nc, W) * sizeof(cx<T>);
         dim3 grid((unsigned)(((long)g.ny * g.nz + W - 1) / W));
         if (prep) {
             auto kern = dct ? k_xfwd_prep<T, true, SH> : k_xfwd_prep<T, false, SH>;
@@ -389,7 +389,7 @@ cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, floa
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
-        const size_t smem = (size_t)nc * W * sizeof(cx<T>);
+        const size_t smem = tile_elems<SH>(nc, W) * sizeof(cx<T>);
         dim3 grid((unsigned)(((long)g.ny * g.nz + W - 1) / W));
         if (blocks_used) *blocks_used = grid.x;
         auto go = [&](auto kern) {

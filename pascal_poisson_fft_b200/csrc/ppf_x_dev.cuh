@@ -120,14 +120,15 @@ __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn
     const bool vec = ((reinterpret_cast<size_t>(f) | reinterpret_cast<size_t>(rs.P) |
                        reinterpret_cast<size_t>(rs.U)) & 15) == 0;
     const long sy = g.pstride_y, sz = g.pstride_z;
+    const int nl = (int)(nlines - line0 < W ? nlines - line0 : W);   // lines of the tile
+    const double* const f0 = f + line0 * nx;   // the tile's lines are contiguous: pair (l, n) at 2 e
+    T* const sr = reinterpret_cast<T*>(s);
 
     for (int e = threadIdx.x; e < E; e += NTH) {
-        const int l = e / nc, n = e - l * nc;
-        const long line = line0 + l;
-        cx<T> z = mk<T>((T)0, (T)0);
-        if (line < nlines) {
-            const double* fl = f + line * nx + 2 * n;
-            double a, b;
+        const int l = div_n<SH>(e, sch), n = e - l * nc;
+        double a = 0.0, b = 0.0;
+        if (l < nl) {
+            const double* fl = f0 + 2 * e;
             if (vec) {
                 const double2 fv = __ldg(reinterpret_cast<const double2*>(fl));
                 a = fv.x;
@@ -159,89 +160,55 @@ __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn
                 b -= (u0 - 2.0 * u1 + xp) * rs.ix2 + (ym1 - 2.0 * u1 + yp1) * rs.iy2 + am * (zm1 - u1) +
                      ap * (zp1 - u1);
             }
-            z = mk<T>((T)a, (T)b);
         }
-        s[tidx<T, SH>(n, l, W)] = z;
+        if constexpr (DCT) {
+            // Makhoul order v = [x0, x2, .., x_{n-2}, x_{n-1}, .., x3, x1]
+            // (cuda_Poisson_DCT_f_pre, fft_3d_poisson.f90:915-935), packed as
+            // complex pairs (v_{2m}, v_{2m+1}) for the half-length FFT: x_2n
+            // is v_n, x_2n+1 is v_{nx-1-n}
+            const int q = nx - 1 - n;
+            sr[2 * tidx<T, SH>(n >> 1, l, W) + (n & 1)] = (T)a;
+            sr[2 * tidx<T, SH>(q >> 1, l, W) + (q & 1)] = (T)b;
+        } else {
+            s[tidx<T, SH>(n, l, W)] = mk<T>((T)a, (T)b);
+        }
     }
     __syncthreads();
 
-    if (DCT) {
-        // Makhoul order v = [x0, x2, .., x_{n-2}, x_{n-1}, .., x3, x1]
-        // (cuda_Poisson_DCT_f_pre, fft_3d_poisson.f90:915-935), packed as
-        // complex pairs (v_{2m}, v_{2m+1}) for the half-length FFT.
-        constexpr int EPT = CT ? (SH::N * SH::W + SH::NT - 1) / SH::NT : 8;
-        cx<T> tmp[EPT];
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) {
-            const int e = threadIdx.x + i * NTH;
-            if (e < E) {
-                const int l = e / nc, m = e - l * nc;
-                const int q0 = 2 * m, q1 = 2 * m + 1;
-                const T v0 = (q0 < nc) ? s[tidx<T, SH>(q0, l, W)].x : s[tidx<T, SH>(nx - 1 - q0, l, W)].y;
-                const T v1 = (q1 < nc) ? s[tidx<T, SH>(q1, l, W)].x : s[tidx<T, SH>(nx - 1 - q1, l, W)].y;
-                tmp[i] = mk<T>(v0, v1);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) {
-            const int e = threadIdx.x + i * NTH;
-            if (e < E) {
-                const int l = e / nc, m = e - l * nc;
-                s[tidx<T, SH>(m, l, W)] = tmp[i];
-            }
-        }
-        __syncthreads();
-    }
-
     tile_fft<T, false, SH>(s, sch, W, lgW, tw_half);
 
-    if (!DCT) {
-        cx<T>* out = reinterpret_cast<cx<T>*>(out_);
-        // R2C split, one pair (k, nc-k) per iteration from z_k and z_{nc-k}
-        const int NP = nc / 2 + 1;
-        for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
-            const int l = e / NP, k = e - l * NP;
-            const long line = line0 + l;
-            if (line >= nlines) continue;
-            const int kc = nc - k;
-            const cx<T> a = s[tidx<T, SH>(k, l, W)];
-            const cx<T> b = s[tidx<T, SH>(k == 0 ? 0 : kc, l, W)];
-            cx<T>* orow = out + line * out_pitch;
-            {
-                const cx<T> zc = conj(b);
-                const cx<T> Ev = (a + zc) * (T)0.5;
-                const cx<T> D = a - zc;
-                const cx<T> O = mk<T>(D.y * (T)0.5, -D.x * (T)0.5);
-                orow[k] = Ev + cmul(ldg(tw_n + k), O);
-            }
-            if (kc != k) {
-                const cx<T> zc = conj(a);
-                const cx<T> Ev = (b + zc) * (T)0.5;
-                const cx<T> D = b - zc;
-                const cx<T> O = mk<T>(D.y * (T)0.5, -D.x * (T)0.5);
-                orow[kc] = Ev + cmul(ldg(tw_n + kc), O);
-            }
-        }
-    } else {
-        // X_k = 2 Re(e^{-i pi k/(2n)} V_k), V_{n-k} = conj(V_k)
-        // (cuda_Poisson_DCT_f_post, fft_3d_poisson.f90:937-969)
-        T* out = reinterpret_cast<T*>(out_);
-        const int Eo = nx * W;
-        for (int e = threadIdx.x; e < Eo; e += NTH) {
-            const int l = e / nx, k = e - l * nx;
-            const long line = line0 + l;
-            if (line >= nlines) continue;
-            const int kap = (k <= nc) ? k : nx - k;
-            const cx<T> zk = s[tidx<T, SH>(kap == nc ? 0 : kap, l, W)];
-            const cx<T> zc = conj(s[tidx<T, SH>(kap == 0 ? 0 : nc - kap, l, W)]);
-            const cx<T> Ev = (zk + zc) * (T)0.5;
-            const cx<T> D = zk - zc;
+    // Real-transform split, one pair (k, nc-k) per iteration from z_k and
+    // z_{nc-k}: V_k = E + w_k O of both.  R2C stores V; the DCT stores
+    // X_k = 2 Re(w V_k) and X_{nx-k} = -2 Im(w V_k), w = e^{-i pi k/(2 nx)}, of
+    // both (V_{nx-k} = conj(V_k); cuda_Poisson_DCT_f_post, fft_3d_poisson.f90:
+    // 937-969): four values from two reads of the tile.
+    const int NP = nc / 2 + 1;
+    for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
+        const int l = div_np<SH>(e, sch), k = e - l * NP;
+        if (l >= nl) continue;
+        const int kc = nc - k;
+        const cx<T> a = s[tidx<T, SH>(k, l, W)];
+        const cx<T> b = s[tidx<T, SH>(k == 0 ? 0 : kc, l, W)];
+        auto half = [&](cx<T> p, cx<T> q, int kk) {
+            const cx<T> zc = conj(q);
+            const cx<T> Ev = (p + zc) * (T)0.5;
+            const cx<T> D = p - zc;
             const cx<T> O = mk<T>(D.y * (T)0.5, -D.x * (T)0.5);
-            cx<T> V = Ev + cmul(ldg(tw_n + kap), O);
-            if (k > nc) V = conj(V);
-            const cx<T> w = ldg(tw_dct + k);
-            out[line * out_pitch + k] = (T)2 * (w.x * V.x - w.y * V.y);
+            return Ev + cmul(ldg(tw_n + kk), O);
+        };
+        if constexpr (!DCT) {
+            cx<T>* orow = reinterpret_cast<cx<T>*>(out_) + (line0 + l) * out_pitch;
+            orow[k] = half(a, b, k);
+            if (kc != k) orow[kc] = half(b, a, kc);
+        } else {
+            T* orow = reinterpret_cast<T*>(out_) + (line0 + l) * out_pitch;
+            auto put = [&](cx<T> V, int kk) {
+                const cx<T> w = ldg(tw_dct + kk);
+                orow[kk] = (T)2 * (w.x * V.x - w.y * V.y);
+                if (kk > 0 && kk < nc) orow[nx - kk] = (T)-2 * (w.x * V.y + w.y * V.x);
+            };
+            put(half(a, b, k), k);
+            if (kc != k) put(half(b, a, kc), kc);
         }
     }
 }
@@ -313,65 +280,45 @@ __device__ __forceinline__ void xinv(const void* __restrict__ in_, long in_pitch
         else P[o] = v;
     };
 
-    if constexpr (!DCT) {
-        // C2R split, one pair (k, nc-k) per iteration: Z_k from (X_k, conj X_{nc-k}),
-        // Z_{nc-k} from (X_{nc-k}, conj X_k)
-        const int NP = nc / 2 + 1;
-        for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
-            const int l = e / NP, k = e - l * NP;
-            const int kc = nc - k;
-            const long line = line0 + l;
-            cx<T> Zk = mk<T>((T)0, (T)0), Zc = Zk;
-            if (line < nlines) {
-                const cx<T>* row = reinterpret_cast<const cx<T>*>(in_) + line * in_pitch;
-                cx<T> xa = row[k], xb = row[kc];
-                if (k == 0) { xa.y = (T)0; xb.y = (T)0; }
-                {
-                    const cx<T> c = conj(xb);
-                    const cx<T> Ev = xa + c, D = xa - c;
-                    const cx<T> O = cmul(D, conj(ldg(tw_n + k)));
-                    Zk = mk<T>(Ev.x - O.y, Ev.y + O.x);
-                }
-                {
-                    const cx<T> c = conj(xa);
-                    const cx<T> Ev = xb + c, D = xb - c;
-                    const cx<T> O = cmul(D, conj(ldg(tw_n + kc)));
-                    Zc = mk<T>(Ev.x - O.y, Ev.y + O.x);
-                }
-            }
-            s[tidx<T, SH>(k, l, W)] = Zk;
-            if (k != 0 && kc != k) s[tidx<T, SH>(kc, l, W)] = Zc;
-        }
-    } else
-    for (int e = threadIdx.x; e < E; e += NTH) {
-        const int l = e / nc, k = e - l * nc;
-        const long line = line0 + l;
-        cx<T> Z = mk<T>((T)0, (T)0);
-        if (line < nlines) {
-            cx<T> xk, xc;
-            if (!DCT) {
-                const cx<T>* row = reinterpret_cast<const cx<T>*>(in_) + line * in_pitch;
-                xk = row[k];
-                xc = conj(row[nc - k]);
-                if (k == 0) { xk.y = (T)0; xc.y = (T)0; }
+    // C2R split, one pair (k, nc-k) per iteration: Z_k from (X_k, conj X_{nc-k}),
+    // Z_{nc-k} from (X_{nc-k}, conj X_k).  DCT: X_j = e^{i pi j/(2 nx)} (C_j -
+    // i C_{nx-j}) of the coefficients C (cuda_Poisson_DCT_b_pre), C_nx = 0.
+    const int NP = nc / 2 + 1;
+    for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
+        const int l = div_np<SH>(e, sch), k = e - l * NP;
+        const int kc = nc - k;
+        cx<T> Zk = mk<T>((T)0, (T)0), Zc = Zk;
+        if (line0 + l < nlines) {
+            cx<T> xa, xb;
+            if constexpr (!DCT) {
+                const cx<T>* row = reinterpret_cast<const cx<T>*>(in_) + (line0 + l) * in_pitch;
+                xa = row[k];
+                xb = row[kc];
             } else {
-                // b_pre: Zs_j = e^{i pi j/(2n)} (X_j - i X_{n-j}), X_n = 0
-                const T* row = reinterpret_cast<const T*>(in_) + line * in_pitch;
-                const int j0 = k, j1 = nc - k;
-                const T a0 = row[j0], b0 = (j0 == 0) ? (T)0 : row[nx - j0];
-                const T a1 = row[j1], b1 = (j1 == 0) ? (T)0 : row[nx - j1];
-                const cx<T> w0 = ldg(tw_dct + j0), w1 = ldg(tw_dct + j1);
+                const T* row = reinterpret_cast<const T*>(in_) + (line0 + l) * in_pitch;
+                const T a0 = row[k], b0 = (k == 0) ? (T)0 : row[nx - k];
+                const T a1 = row[kc], b1 = (k == nc) ? (T)0 : row[nx - kc];
+                const cx<T> w0 = ldg(tw_dct + k), w1 = ldg(tw_dct + kc);
                 const T c0 = w0.x, s0 = -w0.y, c1 = w1.x, s1 = -w1.y;
-                xk = mk<T>(c0 * a0 + s0 * b0, s0 * a0 - c0 * b0);
-                xc = mk<T>(c1 * a1 + s1 * b1, -(s1 * a1 - c1 * b1));
-                if (k == 0) { xk.y = (T)0; xc.y = (T)0; }
+                xa = mk<T>(c0 * a0 + s0 * b0, s0 * a0 - c0 * b0);
+                xb = mk<T>(c1 * a1 + s1 * b1, s1 * a1 - c1 * b1);
             }
-            const cx<T> Ev = xk + xc;
-            const cx<T> D = xk - xc;
-            const cx<T> O = cmul(D, conj(ldg(tw_n + k)));
-            Z = mk<T>(Ev.x - O.y, Ev.y + O.x);
+            if (k == 0) { xa.y = (T)0; xb.y = (T)0; }
+            {
+                const cx<T> c = conj(xb);
+                const cx<T> Ev = xa + c, D = xa - c;
+                const cx<T> O = cmul(D, conj(ldg(tw_n + k)));
+                Zk = mk<T>(Ev.x - O.y, Ev.y + O.x);
+            }
+            {
+                const cx<T> c = conj(xa);
+                const cx<T> Ev = xb + c, D = xb - c;
+                const cx<T> O = cmul(D, conj(ldg(tw_n + kc)));
+                Zc = mk<T>(Ev.x - O.y, Ev.y + O.x);
+            }
         }
-        s[tidx<T, SH>(k, l, W)] = Z;
+        s[tidx<T, SH>(k, l, W)] = Zk;
+        if (k != 0 && kc != k) s[tidx<T, SH>(kc, l, W)] = Zc;
     }
     // ghosted-output offset of each line of the tile, and (GHOST) the offsets
     // of the ghost lines its values are copied to (0: none)
@@ -403,69 +350,47 @@ __device__ __forceinline__ void xinv(const void* __restrict__ in_, long in_pitch
 
     double acc_du = 0.0, acc_u = 0.0, acc_s = 0.0;
     const double mprev = (ACC && mean_prev) ? *mean_prev : 0.0;
-    const int Eo = nx << lgW;
-    if constexpr (!DCT) {
-        // periodic x: outputs x_2n, x_2n+1 are Re, Im of z_n -- two per iteration
-        for (int e = threadIdx.x; e < E; e += NTH) {
-            const int l = e / nc, n = e - l * nc;
-            if (line0 + l >= nlines) continue;
+    // two outputs per iteration: x_2n, x_2n+1 are Re, Im of z_n (periodic x),
+    // or v_n, v_{nx-1-n} of the packed Makhoul order (inverse of the load
+    // order; cuda_Poisson_DCT_b_post, :1013-1033)
+    for (int e = threadIdx.x; e < E; e += NTH) {
+        const int l = div_n<SH>(e, sch), n = e - l * nc;
+        if (line0 + l >= nlines) continue;
+        double x0, x1;
+        if constexpr (!DCT) {
             const cx<T> zv = s[tidx<T, SH>(n, l, W)];
-            const double x0 = (double)zv.x, x1 = (double)zv.y;
-            const long o = line_base[l] + 2 * n;
-            // refinement: u <- u + du - mean(u), the FP64 mean of the previous
-            // iterate (the residual cannot see constants, so the gauge is kept here)
-            double u0 = x0, u1 = x1;
-            if (ACC) {
-                u0 = (src(o) - mprev) + x0;
-                u1 = (src(o + 1) - mprev) + x1;
-            }
-            put(o, u0);
-            put(o + 1, u1);
-            if (GHOST && yz) {
-                // y and z stencil ghosts for the next residual (the reference's
-                // ghost update overwrites them after the last sweep)
-                const long gy = line_gy[l], gz = line_gz[l];
-                if (gy) { put(o + gy, u0); put(o + 1 + gy, u1); }
-                if (gz) { put(o + gz, u0); put(o + 1 + gz, u1); }
-            }
-            if (partials) {
-                // the norms feed the gate after a refinement sweep only
-                if (ACC) {
-                    acc_du += x0 * x0 + x1 * x1;
-                    acc_u += u0 * u0 + u1 * u1;
-                }
-                acc_s += u0 + u1;
-            }
+            x0 = (double)zv.x;
+            x1 = (double)zv.y;
+        } else {
+            const T* sr = reinterpret_cast<const T*>(s);
+            const int q = nx - 1 - n;
+            x0 = (double)sr[2 * tidx<T, SH>(n >> 1, l, W) + (n & 1)];
+            x1 = (double)sr[2 * tidx<T, SH>(q >> 1, l, W) + (q & 1)];
         }
-    } else {
-        for (int e = threadIdx.x; e < Eo; e += NTH) {
-            const int l = e / nx, i = e - l * nx;
-            const long line = line0 + l;
-            if (line >= nlines) continue;
-            int n = i;
-            // inverse Makhoul order (cuda_Poisson_DCT_b_post, :1013-1033)
-            if (DCT) n = (i & 1) ? (nc + ((nx - 1 - i) >> 1)) : (i >> 1);
-            const cx<T> zv = s[tidx<T, SH>(n >> 1, l, W)];
-            const double x = (double)((n & 1) ? zv.y : zv.x);
-            const long o = line_base[l] + i;
-            // refinement: u <- u + du - mean(u), the FP64 mean of the previous
-            // iterate (the residual cannot see constants, so the gauge is kept here)
-            const double un = ACC ? (src(o) - mprev) + x : x;
-            put(o, un);
-            if (GHOST && yz) {
-                // y and z stencil ghosts for the next residual (the reference's
-                // ghost update overwrites them after the last sweep)
-                const long gy = line_gy[l], gz = line_gz[l];
-                if (gy) put(o + gy, un);
-                if (gz) put(o + gz, un);
+        const long o = line_base[l] + 2 * n;
+        // refinement: u <- u + du - mean(u), the FP64 mean of the previous
+        // iterate (the residual cannot see constants, so the gauge is kept here)
+        double u0 = x0, u1 = x1;
+        if (ACC) {
+            u0 = (src(o) - mprev) + x0;
+            u1 = (src(o + 1) - mprev) + x1;
+        }
+        put(o, u0);
+        put(o + 1, u1);
+        if (GHOST && yz) {
+            // y and z stencil ghosts for the next residual (the reference's
+            // ghost update overwrites them after the last sweep)
+            const long gy = line_gy[l], gz = line_gz[l];
+            if (gy) { put(o + gy, u0); put(o + 1 + gy, u1); }
+            if (gz) { put(o + gz, u0); put(o + 1 + gz, u1); }
+        }
+        if (partials) {
+            // the norms feed the gate after a refinement sweep only
+            if (ACC) {
+                acc_du += x0 * x0 + x1 * x1;
+                acc_u += u0 * u0 + u1 * u1;
             }
-            if (partials) {
-                if (ACC) {
-                    acc_du += x * x;
-                    acc_u += un * un;
-                }
-                acc_s += un;
-            }
+            acc_s += u0 + u1;
         }
     }
     if (GHOST) {

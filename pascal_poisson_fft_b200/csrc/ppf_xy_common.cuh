@@ -104,7 +104,7 @@ template <typename T>
 inline bool width_ok(int n, int W)
 {
     if (W < 1 || W > 128 || (W & (W - 1))) return false;
-    return threads_for(n, W) <= 512 && (size_t)n * W * sizeof(cx<T>) <= 200u * 1024u;
+    return threads_for(n, W) <= 512 && (size_t)n * rt_pitch(W) * sizeof(cx<T>) <= 200u * 1024u;
 }
 
 // FFT of the tile with the shape's engine

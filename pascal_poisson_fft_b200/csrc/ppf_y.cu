@@ -327,7 +327,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
-        const size_t smem = (size_t)g.ny * W * sizeof(cx<T>);
+        const size_t smem = tile_elems<SH>(g.ny, W) * sizeof(cx<T>);
         dim3 grid((unsigned)((ncols + W - 1) / W), (unsigned)g.nz);
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
@@ -360,7 +360,7 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
-        const size_t smem = (size_t)g.ny * W * sizeof(cx<T>);
+        const size_t smem = tile_elems<SH>(g.ny, W) * sizeof(cx<T>);
         dim3 grid((unsigned)((ncols + W - 1) / W), (unsigned)g.nz);
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);

@@ -32,14 +32,15 @@ __device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch
     const int NTH = CT ? SH::NT : (int)blockDim.x;
     const int ny = CT ? SH::N : g.ny;
     const int col0 = cblk * W;
-    const cx<T>* inp = in + (long)z * ny * in_pitch;
+    const int nc = ncols - col0 < W ? ncols - col0 : W;   // columns of the tile
+    const cx<T>* inp = in + (long)z * ny * in_pitch + col0;
+    const int ip = (int)in_pitch, op = (int)out_pitch;
     const int E = ny << lgW;
 
     for (int e = threadIdx.x; e < E; e += NTH) {
         const int l = e & (W - 1), y = e >> lgW;
-        const int col = col0 + l;
         cx<T> v = mk<T>((T)0, (T)0);
-        if (col < ncols) v = inp[(long)y * in_pitch + col];
+        if (l < nc) v = inp[y * ip + l];
         int row = y;
         if (KIND == Y_CDCT) row = (y & 1) ? (ny - 1 - (y >> 1)) : (y >> 1);
         s[tidx<T, SH>(row, l, W)] = v;
@@ -48,41 +49,41 @@ __device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch
     tile_fft<T, false, SH>(s, sch, W, lgW, tw_ny);
 
     if (KIND == Y_C2C) {
-        cx<T>* outp = out + (long)z * ny * out_pitch;
+        cx<T>* outp = out + (long)z * ny * out_pitch + col0;
         for (int e = threadIdx.x; e < E; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
-            if (col < ncols) outp[(long)k * out_pitch + col] = s[tidx<T, SH>(k, l, W)];
+            if (l < nc) outp[k * op + l] = s[tidx<T, SH>(k, l, W)];
         }
     } else if (KIND == Y_CDCT) {
-        cx<T>* outp = out + (long)z * ny * out_pitch;
-        for (int e = threadIdx.x; e < E; e += NTH) {
+        // X_k and X_{n-k} from one read of V_k, V_{n-k}: with p = w V_k, q =
+        // conj(w) V_{n-k}, w = e^{-i pi k/(2n)}, X_k = p + q and, as the
+        // twiddle of n - k is -i conj(w), X_{n-k} = i (p - q)
+        cx<T>* outp = out + (long)z * ny * out_pitch + col0;
+        const int Eh = (ny / 2 + 1) << lgW;
+        for (int e = threadIdx.x; e < Eh; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
-            if (col >= ncols) continue;
+            if (l >= nc) continue;
             const cx<T> V = s[tidx<T, SH>(k, l, W)];
             const cx<T> Vp = s[tidx<T, SH>(k == 0 ? 0 : ny - k, l, W)];
             const cx<T> w = ldg(tw_dct + k);
-            cx<T> X;
-            X.x = w.x * (V.x + Vp.x) - w.y * (V.y - Vp.y);
-            X.y = w.x * (V.y + Vp.y) + w.y * (V.x - Vp.x);
-            outp[(long)k * out_pitch + col] = X;
+            const cx<T> p = cmul(w, V), q = cmul(conj(w), Vp);
+            outp[k * op + l] = p + q;
+            if (k > 0 && 2 * k < ny) outp[(ny - k) * op + l] = mk<T>(q.y - p.y, p.x - q.x);
         }
     } else {
         const int my = ny / 2 + 1;
-        cx<T>* outp = out + (long)z * my * out_pitch;
+        cx<T>* outp = out + (long)z * my * out_pitch + 2 * col0;
         const int Eo = my << lgW;
         for (int e = threadIdx.x; e < Eo; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
-            if (col >= ncols) continue;
-            const cx<T> zk = s[tidx<T, SH>(k == ny ? 0 : k, l, W)];
+            if (l >= nc) continue;
+            const cx<T> zk = s[tidx<T, SH>(k, l, W)];
             const cx<T> zc = conj(s[tidx<T, SH>(k == 0 ? 0 : ny - k, l, W)]);
             const cx<T> X1 = (zk + zc) * (T)0.5;
             const cx<T> D = zk - zc;
             const cx<T> X2 = mk<T>(D.y * (T)0.5, -D.x * (T)0.5);
-            outp[(long)k * out_pitch + 2 * col] = X1;
-            outp[(long)k * out_pitch + 2 * col + 1] = X2;
+            outp[k * op + 2 * l] = X1;
+            outp[k * op + 2 * l + 1] = X2;
         }
     }
 }
@@ -107,68 +108,70 @@ __device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch
     // the zero mode's z-average, removed from the (kx,ky) = (0,0) coefficient
     const T shift = (col0 == 0 && dc_shift) ? (T)*dc_shift : (T)0;
 
+    const int nc = ncols - col0 < W ? ncols - col0 : W;   // columns of the tile
+    const int ip = (int)in_pitch, op = (int)out_pitch;
     if (KIND == Y_C2C) {
-        const cx<T>* inp = in + (long)z * ny * in_pitch;
+        const cx<T>* inp = in + (long)z * ny * in_pitch + col0;
         for (int e = threadIdx.x; e < E; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
             cx<T> v = mk<T>((T)0, (T)0);
-            if (col < ncols) v = inp[(long)k * in_pitch + col];
-            if (k == 0 && col == 0) v.x -= shift;
+            if (l < nc) v = inp[k * ip + l];
+            if (e == 0) v.x -= shift;
             s[tidx<T, SH>(k, l, W)] = v;
         }
     } else if (KIND == Y_CDCT) {
-        // Z_k = e^{i pi k/(2n)} (X_k - i X_{n-k}) per real component
+        // Z_k = e^{i pi k/(2n)} (X_k - i X_{n-k}), X_n = 0, per real component
         // (cuda_Poisson_DCT_b_pre, fft_3d_poisson.f90:971-1011), both
-        // components packed into one complex inverse FFT.
-        const cx<T>* inp = in + (long)z * ny * in_pitch;
-        for (int e = threadIdx.x; e < E; e += NTH) {
+        // components packed into one complex inverse FFT: Z_k = conj(w) (X_k -
+        // i X_{n-k}), Z_{n-k} = w (X_k + i X_{n-k}) from one read of the pair
+        const cx<T>* inp = in + (long)z * ny * in_pitch + col0;
+        const int Eh = (ny / 2 + 1) << lgW;
+        for (int e = threadIdx.x; e < Eh; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
-            cx<T> Z = mk<T>((T)0, (T)0);
-            if (col < ncols) {
-                cx<T> X = inp[(long)k * in_pitch + col];
-                if (k == 0 && col == 0) X.x -= shift;
-                const cx<T> Xp = (k == 0) ? mk<T>((T)0, (T)0) : inp[(long)(ny - k) * in_pitch + col];
+            cx<T> Z = mk<T>((T)0, (T)0), Zp = Z;
+            if (l < nc) {
+                cx<T> X = inp[k * ip + l];
+                if (e == 0) X.x -= shift;
+                const cx<T> Xp = (k == 0) ? mk<T>((T)0, (T)0) : inp[(ny - k) * ip + l];
                 const cx<T> w = ldg(tw_dct + k);
-                const T c = w.x, sn = -w.y;
-                const T zax = c * X.x + sn * Xp.x, zay = sn * X.x - c * Xp.x;
-                const T zbx = c * X.y + sn * Xp.y, zby = sn * X.y - c * Xp.y;
-                Z = mk<T>(zax - zby, zay + zbx);
+                Z = cmul(conj(w), mk<T>(X.x + Xp.y, X.y - Xp.x));
+                Zp = cmul(w, mk<T>(X.x - Xp.y, X.y + Xp.x));
             }
             s[tidx<T, SH>(k, l, W)] = Z;
+            if (k > 0 && 2 * k < ny) s[tidx<T, SH>(ny - k, l, W)] = Zp;
         }
     } else {
+        // Z_k = X1_k + i X2_k of the two real columns, Z_{n-k} from the same
+        // pair (both columns' spectra are Hermitian)
         const int my = ny / 2 + 1;
-        const cx<T>* inp = in + (long)z * my * in_pitch;
-        for (int e = threadIdx.x; e < E; e += NTH) {
+        const cx<T>* inp = in + (long)z * my * in_pitch + 2 * col0;
+        const int Eh = my << lgW;
+        for (int e = threadIdx.x; e < Eh; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
-            const int col = col0 + l;
-            cx<T> Z = mk<T>((T)0, (T)0);
-            if (col < ncols) {
-                const int kk = (k <= ny / 2) ? k : ny - k;
-                cx<T> X1 = inp[(long)kk * in_pitch + 2 * col];
-                cx<T> X2 = inp[(long)kk * in_pitch + 2 * col + 1];
-                if (k > ny / 2) { X1 = conj(X1); X2 = conj(X2); }
-                if (k == 0 || k == ny / 2) { X1.y = (T)0; X2.y = (T)0; }
-                if (k == 0 && col == 0) X1.x -= shift;
+            cx<T> Z = mk<T>((T)0, (T)0), Zp = Z;
+            if (l < nc) {
+                cx<T> X1 = inp[k * ip + 2 * l];
+                cx<T> X2 = inp[k * ip + 2 * l + 1];
+                if (k == 0 || 2 * k == ny) { X1.y = (T)0; X2.y = (T)0; }
+                if (e == 0) X1.x -= shift;
                 Z = mk<T>(X1.x - X2.y, X1.y + X2.x);
+                Zp = mk<T>(X1.x + X2.y, X2.x - X1.y);
             }
             s[tidx<T, SH>(k, l, W)] = Z;
+            if (k > 0 && 2 * k < ny) s[tidx<T, SH>(ny - k, l, W)] = Zp;
         }
     }
     __syncthreads();
     tile_fft<T, true, SH>(s, sch, W, lgW, tw_ny);
 
-    cx<T>* outp = out + (long)z * ny * out_pitch;
+    cx<T>* outp = out + (long)z * ny * out_pitch + col0;
     for (int e = threadIdx.x; e < E; e += NTH) {
         const int l = e & (W - 1), i = e >> lgW;
-        const int col = col0 + l;
-        if (col >= ncols) continue;
+        if (l >= nc) continue;
         int n = i;
         // inverse Makhoul order (cuda_Poisson_DCT_b_post, :1013-1033)
         if (KIND == Y_CDCT) n = (i & 1) ? (ny / 2 + ((ny - 1 - i) >> 1)) : (i >> 1);
-        outp[(long)i * out_pitch + col] = s[tidx<T, SH>(n, l, W)];
+        outp[i * op + l] = s[tidx<T, SH>(n, l, W)];
     }
 }
 
