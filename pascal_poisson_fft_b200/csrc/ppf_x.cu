@@ -53,9 +53,12 @@ __global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 
     xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
-// FP64 compile-time tiles: five resident CTAs of SH::NT threads per SM
+// FP64 compile-time tiles: resident CTAs per SM asked of the compiler.  Five
+// of 256 threads (48 registers); of 384 threads two (80): the five once asked
+// left 32 registers and 0.5 to 1 KB of spills a thread.
+constexpr int x64_ctas(int threads) { return threads > 256 ? 2 : 5; }
 template <bool DCT, typename SH, typename T = double>
-__global__ void __launch_bounds__(SH::NT, 5) k_xfwd64(PPF_XFWD_PARAMS)
+__global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PARAMS)
 {
     xfwd<T, DCT, 0, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
@@ -79,9 +82,8 @@ __global__ void __launch_bounds__(512) k_xinv(PPF_XINV_PARAMS)
     xinv<T, DCT, ACC, GHOST, SH, UK>(PPF_XINV_ARGS);
 }
 
-// FP64 compile-time tiles: five resident CTAs of SH::NT threads per SM
 template <bool DCT, typename SH, typename T = double>
-__global__ void __launch_bounds__(SH::NT, 5) k_xinv64(PPF_XINV_PARAMS)
+__global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xinv64(PPF_XINV_PARAMS)
 {
     xinv<T, DCT, false, false, SH>(PPF_XINV_ARGS);
 }

@@ -244,9 +244,10 @@ __global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* __restrict__
 }
 
 // FP64 tiles (half width, 256 threads): three resident CTAs per SM, which
-// bounds the registers to 85 a thread
+// bounds the registers to 85 a thread; two of the 384-thread shapes (three
+// left 56 registers and 200 bytes of spills)
 template <bool INV, typename SH>
-__global__ void __launch_bounds__(SH::NT, 3) k_y_c2c_pipe64(const cx<double>* __restrict__ in, long in_pitch,
+__global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 3) k_y_c2c_pipe64(const cx<double>* __restrict__ in, long in_pitch,
                                                            cx<double>* __restrict__ out, long out_pitch, int ncols,
                                                            int nz, const cx<double>* __restrict__ tw,
                                                            const double* __restrict__ dc_shift,
