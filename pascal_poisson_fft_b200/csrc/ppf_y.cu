@@ -27,8 +27,25 @@
 
 namespace ppf {
 
+// Tile shape of the FP64 y kernels.  FP64 tiles of 512-thread shapes
+// are halved (W/2 columns, 256 threads): two 32 KB buffers per CTA let three
+// CTAs share an SM, with 8 complex values per thread.
+template <typename T, typename SH>
+struct PipeShape {
+    using type = SH;
+};
+template <int N, int W, int... RS>
+struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
+    using type = ShapeCT<N, W / 2, 256, RS...>;
+};
+
+// resident CTAs asked of the compile-time y tiles of the DCT and packed-real
+// kinds
+template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
+template <typename SH> constexpr int y_ctas = !SH::CT ? 0 : SH::NT <= 256 ? 4 : 2;
+
 template <typename T, int KIND, typename SH>
-__global__ void __launch_bounds__(512) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const int* __restrict__ skip)
@@ -38,7 +55,7 @@ __global__ void __launch_bounds__(512) k_yfwd(const cx<T>* __restrict__ in, long
 }
 
 template <typename T, int KIND, typename SH>
-__global__ void __launch_bounds__(512) k_yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const double* __restrict__ dc_shift, const int* __restrict__ skip)
@@ -256,18 +273,6 @@ __global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 3) k_y_c2c_pipe64(c
     y_c2c_pipe<double, INV, SH, false>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip);
 }
 
-// Tile shape of the pipelined y kernel.  FP64 tiles of 512-thread shapes
-// are halved (W/2 columns, 256 threads): two 32 KB buffers per CTA let three
-// CTAs share an SM, with 8 complex values per thread.
-template <typename T, typename SH>
-struct PipeShape {
-    using type = SH;
-};
-template <int N, int W, int... RS>
-struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
-    using type = ShapeCT<N, W / 2, 256, RS...>;
-};
-
 template <typename T, bool INV, typename SH>
 cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch, int ncols, int nz,
                               const cx<T>* tw, const double* dc_shift, const int* skip_flag, cudaStream_t st,
@@ -324,7 +329,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
 {
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
-        using SH = decltype(sh);
+        using SH = typename PipeShape<T, decltype(sh)>::type;
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
@@ -339,7 +344,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
-                err = launch_y_c2c_pipe<T, false, typename PipeShape<T, SH>::type>(in, in_pitch, out, out_pitch,
+                err = launch_y_c2c_pipe<T, false, SH>(in, in_pitch, out, out_pitch,
                                                                                   ncols, g.nz, tw_ny, nullptr,
                                                                                   skip_flag, st, err_bits);
             else go(k_yfwd<T, Y_C2C, SH>);
@@ -357,7 +362,7 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
 {
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
-        using SH = decltype(sh);
+        using SH = typename PipeShape<T, decltype(sh)>::type;
         int W, threads;
         shape_geom<T, SH>(sch, W, threads);
         if (threads > 512) { err = cudaErrorInvalidConfiguration; return; }
@@ -372,7 +377,7 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
-                err = launch_y_c2c_pipe<T, true, typename PipeShape<T, SH>::type>(in, in_pitch, out, out_pitch,
+                err = launch_y_c2c_pipe<T, true, SH>(in, in_pitch, out, out_pitch,
                                                                                  ncols, g.nz, tw_ny, dc_shift,
                                                                                  skip_flag, st, err_bits);
             else go(k_yinv<T, Y_C2C, SH>);
