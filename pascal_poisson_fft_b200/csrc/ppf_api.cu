@@ -710,8 +710,7 @@ int ppf_stage_times(ppf_plan* plan, double* ms, int* launches)
             float t = 0.f;
             cudaEventElapsedTime(&t, prev, m.second);
             ms[m.first] += t;
-            // ghosts launch one kernel per axis; every other stage one kernel
-            launches[m.first] += (m.first == 7) ? 3 : 1;
+            launches[m.first] += 1;
         }
         prev = m.second;
     }
