@@ -437,7 +437,7 @@ int plan_alloc_work(ppf_plan* p)
 // residual and the accumulate read it (U_ACC: from p->U).
 template <typename T>
 int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulate, const int* skip,
-             cudaStream_t st, int uk = U_P, const double* dx3 = nullptr, const double* dmx3 = nullptr)
+             LStream st, int uk = U_P, const double* dx3 = nullptr, const double* dmx3 = nullptr)
 {
     const cx<T>* tw = reinterpret_cast<const cx<T>*>(p->tw);
     const cx<T>* txh = tw + p->tw_off[0];
@@ -487,7 +487,7 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
         zp.f32 = sizeof(T) == 4; zp.cyclic = p->g.pz;
     }
     cudaError_t e = launch_xfwd<T>(p->xdct, f, resid ? &rs : nullptr, p->g, p->A, p->a_pitch, p->sx, txh, txn, txd,
-                                   skip, st, resid ? nullptr : &zp);
+                                   skip, resid ? st : LStream(st.s), resid ? nullptr : &zp);
     if (e != cudaSuccess) return cuda_fail(e, "x forward");
     if (!resid && z.lowk_list) {
         // the FP64 low-|k| set of this solve (flags[3], zeroed with the
@@ -500,16 +500,19 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
     const long a_cp = p->xdct ? p->a_pitch / 2 : p->a_pitch;
     const long b_cp = (p->xdct && p->ydct) ? p->b_pitch / 2 : p->b_pitch;
     e = launch_yfwd<T>(p->ykind, reinterpret_cast<const cx<T>*>(p->A), a_cp, reinterpret_cast<cx<T>*>(p->B), b_cp,
-                       p->ycols, p->g, p->sy, tyn, tyd, skip, st, p->flags + 2);
+                       p->ycols, p->g, p->sy, tyn, tyd, skip, (!resid && z.lowk_list) ? LStream(st.s) : st,
+                       p->flags + 2);
     if (e != cudaSuccess) return cuda_fail(e, "y forward");
     mark(p, 2, st);
-    const ZStreams zs{ st, p->aux, p->ev_fork, p->ev_join };
+    // the z solve of FP32 spectra without tables forks to the auxiliary stream
+    const bool fork = sizeof(T) == 4 && !z.tab;
+    const ZStreams zs{ fork ? LStream(st.s) : st, p->aux, p->ev_fork, p->ev_join };
     e = p->cplx ? launch_tdma_z<T, true>(p->B, z, skip, p->flags + 2, zs)
                 : launch_tdma_z<T, false>(p->B, z, skip, p->flags + 2, zs);
     if (e != cudaSuccess) return cuda_fail(e, "z tridiagonal");
     mark(p, 3, st);
     e = launch_yinv<T>(p->ykind, reinterpret_cast<const cx<T>*>(p->B), b_cp, reinterpret_cast<cx<T>*>(p->A), a_cp,
-                       p->ycols, p->g, p->sy, tyn, tyd, p->scal + 4, skip, st, p->flags + 2);
+                       p->ycols, p->g, p->sy, tyn, tyd, p->scal + 4, skip, fork ? LStream(st.s) : st, p->flags + 2);
     if (e != cudaSuccess) return cuda_fail(e, "y inverse");
     mark(p, 4, st);
     // the mixed path keeps the stencil's ghost cells current for its residual
@@ -523,13 +526,27 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
 }
 
 int solve_impl(ppf_plan* p, const double* f, double* P, const double* dmx1, const double* dmx2,
-               const double* dmx3, const double* dx3, cudaStream_t st)
+               const double* dmx3, const double* dx3, cudaStream_t stream)
 {
     if (!p) return fail(PPF_ERR_INVALID, "null plan");
     if (!f || !P || !dmx1 || !dmx2 || !dmx3 || !dx3) return fail(PPF_ERR_INVALID, "null array argument");
     int cur = -1;
     PPF_CK(cudaGetDevice(&cur));
     if (cur != p->dev) return fail(PPF_ERR_STATE, "plan was created on device %d, current device is %d", p->dev, cur);
+    // Overlapped launches (LStream) of a solve on its own: 10 us of a small
+    // solve's launches (64^3 44 -> 35, 256 x 256 x 128 206 -> 196, 384 x 256 x
+    // 100 257 -> 250).  FP64 grids above 12 M cells do without: the next
+    // kernel's blocks, resident early, disturb the persistent y tiles and the
+    // z sweep (256^3 379 -> 390, 512^3 2554 -> 2932); FP32 is the same or
+    // faster at every size.  A captured graph launches its nodes fast as it
+    // is, the problems of a batch would hold one another's blocks back, and
+    // stage timing puts events between kernels.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PPF_CK(cudaStreamIsCapturing(stream, &cap));
+    const long cells = (long)p->g.nx * p->g.ny * p->g.nz;
+    const bool overlap = cap == cudaStreamCaptureStatusNone && !p->batch_member && !p->timing &&
+                         (p->elem == 4 || cells <= 12000000);
+    const LStream st(stream, overlap);
     mark(p, -1, st);
     cudaError_t e;
     int rc;

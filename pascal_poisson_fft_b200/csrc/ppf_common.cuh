@@ -81,6 +81,48 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// Programmatic dependent launch: a solve's kernels on one stream are launched
+// with this allowed, so that the next kernel's blocks are resident and past
+// their launch latency when the previous kernel ends.  Every such kernel
+// begins with pdl_enter(): it waits for the whole previous kernel (and so,
+// each having waited for its own, for all before it) before it touches
+// memory, then lets the next kernel's blocks in.  Without the launch
+// attribute both instructions do nothing.  A solve's first launch waits for
+// its predecessor as usual, and its last kernel only waits (pdl_wait): what
+// runs before and after a solve sees ordinary stream order.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter()
+{
+    pdl_wait();
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// the stream of a launch, and whether the launch may overlap the end of the
+// previous kernel on it (which must then be followed by nothing but kernels
+// that begin with pdl_enter)
+struct LStream {
+    cudaStream_t s;
+    bool pdl;
+    LStream(cudaStream_t st = nullptr, bool p = false) : s(st), pdl(p) {}
+    operator cudaStream_t() const { return s; }
+};
+
+template <typename... P, typename... A>
+inline cudaError_t launch_on(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, const LStream& st, A&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st.s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = st.pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Per-axis FFT schedule: complex length n = prod(radix[0..npass)).
 struct FftSched {
     int n;

@@ -66,6 +66,7 @@ __device__ __forceinline__ GhostAxis ghost_axis_of(const GhostArgs& g, int d, in
 
 __global__ void __launch_bounds__(256) k_ghosts(const __grid_constant__ GhostArgs g)
 {
+    pdl_wait();
     const long total = g.count[0] + g.count[1] + g.count[2];
     for (long q = threadIdx.x + (long)blockIdx.x * blockDim.x; q < total; q += (long)blockDim.x * gridDim.x) {
         int c[3];
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(256) k_ghosts(const __grid_constant__ GhostArg
 }
 
 cudaError_t launch_ghosts(double* P, const Geom& g, const double* dmx1, const double* dmx2, const double* dmx3,
-                          cudaStream_t st, int zfaces)
+                          LStream st, int zfaces)
 {
     GhostArgs a{};
     a.P = P;
@@ -125,23 +126,21 @@ cudaError_t launch_ghosts(double* P, const Geom& g, const double* dmx1, const do
     a.count[1] = 2L * g.nx * (g.nz + 2);
     a.count[2] = (long)((zfaces & 1) + (zfaces >> 1)) * g.nx * g.ny;
     const long want = (a.count[0] + a.count[1] + a.count[2] + 255) / 256;
-    k_ghosts<<<(unsigned)std::min(want, 148L * 64), 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_on(k_ghosts, dim3((unsigned)std::min(want, 148L * 64)), 256, 0, st, a);
 }
 
 __global__ void __launch_bounds__(512) k_sweep_gate(const double* __restrict__ partials, long nblocks, double ncell,
                                                     double* mean_prev, int* skip, int* sweeps_done, double* last_rel,
                                                     double tol, int initial)
 {
+    pdl_enter();
     sweep_gate(partials, nblocks, ncell, mean_prev, skip, sweeps_done, last_rel, tol, initial);
 }
 
 cudaError_t launch_sweep_gate(const double* partials, long nblocks, double ncell, double* mean_prev, int* skip_flag,
-                              int* sweeps_done, double* last_rel, double tol, int initial, cudaStream_t st)
+                              int* sweeps_done, double* last_rel, double tol, int initial, LStream st)
 {
-    k_sweep_gate<<<1, 512, 0, st>>>(partials, nblocks, ncell, mean_prev, skip_flag, sweeps_done, last_rel, tol,
-                                    initial);
-    return cudaGetLastError();
+    return launch_on(k_sweep_gate, dim3(1), 512, 0, st, partials, nblocks, ncell, mean_prev, skip_flag, sweeps_done, last_rel, tol, initial);
 }
 
 }  // namespace ppf

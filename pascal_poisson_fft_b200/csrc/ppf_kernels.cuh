@@ -29,19 +29,19 @@ template <typename T>
 cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const Geom& g,
                         void* out, long out_pitch, const FftSched& sch,
                         const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st, const struct ZPrep* prep = nullptr);
+                        const int* skip_flag, LStream st, const struct ZPrep* prep = nullptr);
 
 template <typename T>
 cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch,
                         int ncols, const Geom& g, const FftSched& sch,
-                        const cx<T>* tw_ny, const cx<T>* tw_dct, const int* skip_flag, cudaStream_t st,
+                        const cx<T>* tw_ny, const cx<T>* tw_dct, const int* skip_flag, LStream st,
                         int* err = nullptr);
 
 template <typename T>
 cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch,
                         int ncols, const Geom& g, const FftSched& sch,
                         const cx<T>* tw_ny, const cx<T>* tw_dct, const double* dc_shift,
-                        const int* skip_flag, cudaStream_t st, int* err = nullptr);
+                        const int* skip_flag, LStream st, int* err = nullptr);
 
 // Where the x inverse reads and writes the iterate of a mixed solve.  The
 // first iterate is made of FP32 values, so when a refinement sweep follows it
@@ -57,7 +57,7 @@ template <typename T>
 cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, float* U, int ukind, const Geom& g,
                         bool accumulate, bool stencil_ghosts, double* partials, const double* mean_prev,
                         const FftSched& sch, const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st, long* blocks_used = nullptr, int* err = nullptr);
+                        const int* skip_flag, LStream st, long* blocks_used = nullptr, int* err = nullptr);
 
 // upper bound of the blocks launch_xinv uses for geometry g (one per tile;
 // size of the partials array / 3); the launch reports the blocks it used
@@ -129,7 +129,7 @@ inline unsigned zprep_blocks(const ZPrep& q, int threads)
 }
 inline size_t zprep_smem(int nz) { return sizeof(double) * (3 * (size_t)nz + 32); }
 // the preparation in a launch of its own (a solve without tables)
-cudaError_t launch_zprep(const ZPrep& q, cudaStream_t st);
+cudaError_t launch_zprep(const ZPrep& q, LStream st);
 // doubles of the tables
 inline long ztab_doubles(int nz, long tplane, int cyclic, bool fp32)
 {
@@ -148,7 +148,7 @@ int* tdma_z_lowk_list(double* ckpt, int nz, long plane, int cyclic);
 // systems run on aux (forked from and joined back to st through the two
 // events) when aux is given, else on st after the bulk
 struct ZStreams {
-    cudaStream_t st;
+    LStream st;
     cudaStream_t aux;
     cudaEvent_t fork, join;
 };
@@ -158,13 +158,13 @@ cudaError_t launch_tdma_z(void* data, const ZSys& z, const int* skip_flag, int* 
 
 // the low-|k| system list of a mixed or FP32 solve (z.lowk_list), once per
 // solve before its first z solve; a no-op where the list is not used
-cudaError_t launch_lowk_list(const ZSys& z, cudaStream_t st);
+cudaError_t launch_lowk_list(const ZSys& z, LStream st);
 
 // ---- ghost cells (ppf_ghost.cu) ----
 // zfaces: z faces to fill (1 lower, 2 upper; 3 for a whole domain, the
 // ends of a z slab that are global walls for a slab)
 cudaError_t launch_ghosts(double* P, const Geom& g, const double* dmx1, const double* dmx2,
-                          const double* dmx3, cudaStream_t st, int zfaces = 3);
+                          const double* dmx3, LStream st, int zfaces = 3);
 
 // ---- field IO of the example drivers (ppf_post.cu) ----
 // ghost update of a ghosted field: walls != 0, the solve's (Neumann
@@ -200,7 +200,7 @@ cudaError_t launch_tdma_update(const double* a, const double* c, double* d, cons
 // the gate (skip_flag) below tol.
 cudaError_t launch_sweep_gate(const double* partials, long nblocks, double ncell, double* mean_prev,
                               int* skip_flag, int* sweeps_done, double* last_rel, double tol, int initial,
-                              cudaStream_t st);
+                              LStream st);
 
 // ---- transpose of the solve and z-metric gradient (ppf_adjoint.cu) ----
 // per-level reductions run over nchunk blocks of `chunk` cells of a plane

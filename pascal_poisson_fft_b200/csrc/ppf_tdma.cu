@@ -85,6 +85,7 @@ template <typename T, typename A, bool CPLX, int MODE, bool CYC>
 __global__ void __launch_bounds__(TPB) k_thomas_z(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
                                                   int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     using E = typename Elem<T, CPLX>::type;
     E* data = reinterpret_cast<E*>(data_);
@@ -636,7 +637,7 @@ __global__ void __launch_bounds__(ZStream::NT, 1)
 // rows the tensor map can describe, shared memory for at least three
 // boxes); *used false: the caller takes k_thomas_fast.
 template <bool CPLX>
-cudaError_t launch_stream(void* data, const ZSys& z, const int* skip, int* err, cudaStream_t st, bool* used)
+cudaError_t launch_stream(void* data, const ZSys& z, const int* skip, int* err, LStream st, bool* used)
 {
     using S = ZStream;
     constexpr int EC = CPLX ? 2 : 1;
@@ -682,6 +683,7 @@ template <bool CPLX, bool PREF>
 __global__ void __launch_bounds__(TPB) k_thomas_exact(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
                                                       int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     extern __shared__ double zl[];     // am[nz], ap[nz], s[nz] = -am - ap
     const int nz = z.nz;
@@ -1277,6 +1279,7 @@ template <typename T, bool CPLX, bool KEEP>
 __global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
                                                         int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     constexpr int SH = CPLX ? 1 : 0;
     extern __shared__ double tab_raw[];
@@ -1341,6 +1344,7 @@ template <bool CPLX, bool KEEP>
 __global__ void __launch_bounds__(TAB_TPB) k_thomas_tab_cyc(void* __restrict__ data_, ZSys z,
                                                             const int* __restrict__ skip, int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     using X = Exact;
     constexpr int SH = CPLX ? 1 : 0, C = TAB_C;
@@ -1403,7 +1407,7 @@ __global__ void __launch_bounds__(TAB_TPB) k_thomas_tab_cyc(void* __restrict__ d
 }
 
 template <typename T, bool CPLX>
-cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, cudaStream_t st)
+cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, LStream st)
 {
     const unsigned nb = (unsigned)(((z.plane << (CPLX ? 1 : 0)) + TAB_TPB - 1) / TAB_TPB);
     const unsigned grid = sizeof(T) == 4 ? 2 * nb : nb;
@@ -1421,8 +1425,7 @@ cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, cud
             const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
         }
-        kern<<<grid, TAB_TPB, smem, st>>>(data, z, skip, err);
-        return cudaGetLastError();
+        return launch_on(kern, dim3(grid), TAB_TPB, smem, st, data, z, skip, err);
     };
     if constexpr (sizeof(T) == 8)
         if (z.cyclic)
@@ -1435,9 +1438,8 @@ cudaError_t launch_z(double*, const ZSys& z, void* data, const int* skip, int* e
 {
     if (z.tab) return launch_tab<double, CPLX>(z, data, skip, err, zs.st);
     dim3 grid((unsigned)((z.plane + TPB - 1) / TPB));  // pitch * my systems incl. padding columns
-    if (CYC) k_thomas_z<double, Exact, CPLX, 0, CYC><<<grid, TPB, 0, zs.st>>>(data, z, skip, err);
-    else k_thomas_exact<CPLX, true><<<grid, TPB, 3 * sizeof(double) * z.nz, zs.st>>>(data, z, skip, err);
-    return cudaGetLastError();
+    if (CYC) return launch_on(k_thomas_z<double, Exact, CPLX, 0, CYC>, grid, TPB, 0, zs.st, data, z, skip, err);
+    return launch_on(k_thomas_exact<CPLX, true>, grid, TPB, 3 * sizeof(double) * z.nz, zs.st, data, z, skip, err);
 }
 // FP32 data: the bulk in FP32 and, concurrently on the auxiliary stream when
 // one is given, the few low-|k| systems in FP64 (a short grid-wide launch
@@ -1447,9 +1449,9 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
 {
     if (z.tab) return launch_tab<float, CPLX>(z, data, skip, err, zs.st);
     dim3 grid((unsigned)((z.plane + TPB - 1) / TPB));
-    cudaStream_t lo = zs.st;
+    cudaStream_t lo = zs.st.s;
     if (zs.aux) {
-        cudaError_t e = cudaEventRecord(zs.fork, zs.st);
+        cudaError_t e = cudaEventRecord(zs.fork, zs.st.s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(zs.aux, zs.fork, 0);
         if (e != cudaSuccess) return e;
         lo = zs.aux;
@@ -1475,28 +1477,28 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
     }
     bool streamed = false;
     if (!CYC && z.ckpt_f) {
-        const cudaError_t e = launch_stream<CPLX>(data, z, skip, err, zs.st, &streamed);
+        const cudaError_t e = launch_stream<CPLX>(data, z, skip, err, zs.st.s, &streamed);
         if (e != cudaSuccess) return e;
     }
     if (!streamed) {
         if (CYC || !z.ckpt_f || z.plane >= (1L << 31) / 4)
-            k_thomas_z<float, Fast, CPLX, 1, CYC><<<grid, TPB, 0, zs.st>>>(data, z, skip, err);
+            k_thomas_z<float, Fast, CPLX, 1, CYC><<<grid, TPB, 0, zs.st.s>>>(data, z, skip, err);
         else
-            k_thomas_fast<CPLX><<<grid, TPB, sizeof(float4) * z.nz, zs.st>>>(data, z, skip, err);
+            k_thomas_fast<CPLX><<<grid, TPB, sizeof(float4) * z.nz, zs.st.s>>>(data, z, skip, err);
     }
     if (zs.aux) {
         cudaError_t e = cudaEventRecord(zs.join, zs.aux);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(zs.st, zs.join, 0);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(zs.st.s, zs.join, 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
 }  // namespace
 
-cudaError_t launch_lowk_list(const ZSys& z, cudaStream_t st)
+cudaError_t launch_lowk_list(const ZSys& z, LStream st)
 {
     if (!lowk_listed(z)) return cudaSuccess;
-    k_lowk_list<<<(unsigned)((z.plane + 255) / 256), 256, 0, st>>>(z);
+    k_lowk_list<<<(unsigned)((z.plane + 255) / 256), 256, 0, st.s>>>(z);
     return cudaGetLastError();
 }
 
@@ -1783,14 +1785,14 @@ cudaError_t launch_tdma_update(const double* a, const double* c, double* d, cons
 // the z preparation alone (one block: no tables)
 __global__ void __launch_bounds__(256) k_zprep(const __grid_constant__ ZPrep zp)
 {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char prep_raw[];
     zprep(zp, blockIdx.x, reinterpret_cast<double*>(prep_raw));
 }
 
-cudaError_t launch_zprep(const ZPrep& zp, cudaStream_t st)
+cudaError_t launch_zprep(const ZPrep& zp, LStream st)
 {
-    k_zprep<<<1, 256, zprep_smem(zp.nz), st>>>(zp);
-    return cudaGetLastError();
+    return launch_on(k_zprep, dim3(1), 256, zprep_smem(zp.nz), st, zp);
 }
 
 }  // namespace ppf

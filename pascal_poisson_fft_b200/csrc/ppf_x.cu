@@ -37,6 +37,7 @@ template <typename T, bool DCT, typename SH>
 __global__ void __launch_bounds__(512, (SH::CT && SH::NT <= 256) ? 2 : 0)
     k_xfwd_prep(PPF_XFWD_PARAMS, const __grid_constant__ ZPrep zp, unsigned nprep)
 {
+    pdl_enter();
     if (blockIdx.x < nprep) {
         extern __shared__ __align__(16) unsigned char prep_raw[];
         zprep(zp, blockIdx.x, reinterpret_cast<double*>(prep_raw));
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(512, (SH::CT && SH::NT <= 256) ? 2 : 0)
 template <typename T, bool DCT, int RESID, typename SH>
 __global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 : 0) k_xfwd(PPF_XFWD_PARAMS)
 {
+    pdl_enter();
     xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
@@ -60,6 +62,7 @@ constexpr int x64_ctas(int threads) { return threads > 256 ? 2 : 5; }
 template <bool DCT, typename SH, typename T = double>
 __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PARAMS)
 {
+    pdl_enter();
     xfwd<T, DCT, 0, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
@@ -79,12 +82,14 @@ __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PA
 template <typename T, bool DCT, bool ACC, bool GHOST, typename SH, int UK = U_P>
 __global__ void __launch_bounds__(512) k_xinv(PPF_XINV_PARAMS)
 {
+    pdl_enter();
     xinv<T, DCT, ACC, GHOST, SH, UK>(PPF_XINV_ARGS);
 }
 
 template <bool DCT, typename SH, typename T = double>
 __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xinv64(PPF_XINV_PARAMS)
 {
+    pdl_enter();
     xinv<T, DCT, false, false, SH>(PPF_XINV_ARGS);
 }
 
@@ -118,6 +123,7 @@ __global__ void __launch_bounds__(SH::NT, (SH::N <= 128) ? 2 : SH::N == 384 ? 3 
                                                      const cx<T>* __restrict__ tw_n, const int* __restrict__ skip,
                                                      int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     constexpr int NC = SH::N, W = SH::W, NT = SH::NT;
     constexpr int NR = NC + 1;
@@ -311,7 +317,7 @@ __global__ void __launch_bounds__(SH::NT, (SH::N <= 128) ? 2 : SH::N == 384 ? 3 
 template <typename T>
 cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const Geom& g, void* out, long out_pitch,
                         const FftSched& sch, const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st, const ZPrep* prep)
+                        const int* skip_flag, LStream st, const ZPrep* prep)
 {
     const int nc = g.nx / 2;
     ResidIn rs{};
@@ -336,17 +342,15 @@ cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const G
             const unsigned nprep = zprep_blocks(*prep, threads);
             err = set_smem(kern, psmem);
             if (err != cudaSuccess) return;
-            kern<<<grid.x + nprep, threads, psmem, st>>>(f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n,
+            err = launch_on(kern, dim3(grid.x + nprep), threads, psmem, st, f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n,
                                                         tw_dct, skip_flag, *prep, nprep);
-            err = cudaGetLastError();
             return;
         }
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
             if (err != cudaSuccess) return;
-            kern<<<grid, threads, smem, st>>>(f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n, tw_dct,
+            err = launch_on(kern, grid, threads, smem, st, f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n, tw_dct,
                                               skip_flag);
-            err = cudaGetLastError();
         };
         if constexpr (SH::CT && sizeof(T) == 8) {
             if (!resid) {
@@ -377,7 +381,7 @@ template <typename T>
 cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, float* U, int ukind, const Geom& g,
                         bool accumulate, bool stencil_ghosts, double* partials, const double* mean_prev,
                         const FftSched& sch, const cx<T>* tw_half, const cx<T>* tw_n, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st, long* blocks_used, int* err_bits)
+                        const int* skip_flag, LStream st, long* blocks_used, int* err_bits)
 {
     const int nc = g.nx / 2;
     int* const ebits = err_bits;
@@ -397,9 +401,8 @@ cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, floa
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
             if (err != cudaSuccess) return;
-            kern<<<grid, threads, smem, st>>>(in, in_pitch, P, U, g, partials, mean_prev, sch, W, ilog2i(W), tw_half,
+            err = launch_on(kern, grid, threads, smem, st, in, in_pitch, P, U, g, partials, mean_prev, sch, W, ilog2i(W), tw_half,
                                               tw_n, tw_dct, skip_flag);
-            err = cudaGetLastError();
         };
         if constexpr (SH::CT && sizeof(T) == 4) {
             if (!dct) {  // pipelined FP32 tiles
@@ -411,9 +414,8 @@ cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, floa
                     if (err == cudaSuccess) err = persistent_grid(kern, SH::NT, psmem, (long)grid.x, &pgrid);
                     if (err != cudaSuccess) return;
                     if (blocks_used) *blocks_used = pgrid;
-                    kern<<<pgrid, SH::NT, psmem, st>>>(reinterpret_cast<const cx<T>*>(in), in_pitch, P, U, g,
+                    err = launch_on(kern, dim3(pgrid), SH::NT, psmem, st, reinterpret_cast<const cx<T>*>(in), in_pitch, P, U, g,
                                                       partials, mean_prev, tw_half, tw_n, skip_flag, ebits);
-                    err = cudaGetLastError();
                 };
                 // bulk row copies where every row starts on a 16-byte boundary
                 // and the pitch holds the NC + 2 values a copy reads
@@ -489,12 +491,12 @@ long xinv_blocks(const Geom& g, const FftSched& sch)
 #if PPF_FWD
 template cudaError_t launch_xfwd<PPF_REAL>(bool, const double*, const ResidIn*, const Geom&, void*, long,
                                            const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*,
-                                           const cx<PPF_REAL>*, const int*, cudaStream_t, const ZPrep*);
+                                           const cx<PPF_REAL>*, const int*, LStream, const ZPrep*);
 #else
 template long xinv_blocks<PPF_REAL>(const Geom&, const FftSched&);
 template cudaError_t launch_xinv<PPF_REAL>(bool, const void*, long, double*, float*, int, const Geom&, bool, bool,
                                            double*, const double*, const FftSched&, const cx<PPF_REAL>*,
-                                           const cx<PPF_REAL>*, const cx<PPF_REAL>*, const int*, cudaStream_t, long*,
+                                           const cx<PPF_REAL>*, const cx<PPF_REAL>*, const int*, LStream, long*,
                                            int*);
 #endif
 

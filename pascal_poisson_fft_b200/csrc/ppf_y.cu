@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>*
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const int* __restrict__ skip)
 {
+    pdl_enter();
     yfwd<T, KIND, SH>(in, in_pitch, out, out_pitch, ncols, g, sch, Wrt, lgWrt, tw_ny, tw_dct, skip, blockIdx.x,
                       blockIdx.y);
 }
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yinv(const cx<T>*
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const double* __restrict__ dc_shift, const int* __restrict__ skip)
 {
+    pdl_enter();
     yinv<T, KIND, SH>(in, in_pitch, out, out_pitch, ncols, g, sch, Wrt, lgWrt, tw_ny, tw_dct, dc_shift, skip,
                       blockIdx.x, blockIdx.y);
 }
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(SH::NT, 1) k_y_c2c_tma(const __grid_constant__
                                                      const double* __restrict__ dc_shift,
                                                      const int* __restrict__ skip, int* __restrict__ err)
 {
+    pdl_enter();
     if (skip && *skip) return;
     using T = float;
     constexpr int N = SH::N, W = SH::W;
@@ -257,6 +260,7 @@ __global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* __restrict__
                                                       const double* __restrict__ dc_shift,
                                                       const int* __restrict__ skip)
 {
+    pdl_enter();
     y_c2c_pipe<T, INV, SH, PAIR>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip);
 }
 
@@ -270,12 +274,13 @@ __global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 3) k_y_c2c_pipe64(c
                                                            const double* __restrict__ dc_shift,
                                                            const int* __restrict__ skip)
 {
+    pdl_enter();
     y_c2c_pipe<double, INV, SH, false>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip);
 }
 
 template <typename T, bool INV, typename SH>
 cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch, int ncols, int nz,
-                              const cx<T>* tw, const double* dc_shift, const int* skip_flag, cudaStream_t st,
+                              const cx<T>* tw, const double* dc_shift, const int* skip_flag, LStream st,
                               int* err)
 {
     if constexpr (sizeof(T) == 4 && PairWidth<SH::W>::value && PPF_Y_TMA_W(SH::W) &&
@@ -296,9 +301,8 @@ cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long o
             unsigned grid = 0;
             e = persistent_grid(kern, SH::NT, smem, tiles, &grid);
             if (e != cudaSuccess) return e;
-            kern<<<grid, SH::NT, smem, st>>>(map, reinterpret_cast<cx<float>*>(out), out_pitch, ncols, nz,
+            return launch_on(kern, dim3(grid), SH::NT, smem, st, map, reinterpret_cast<cx<float>*>(out), out_pitch, ncols, nz,
                                             reinterpret_cast<const cx<float>*>(tw), dc_shift, skip_flag, err);
-            return cudaGetLastError();
         }
     }
     // paired passes where the tile is 16 FP32 columns and every column pair
@@ -318,14 +322,13 @@ cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long o
     unsigned grid = 0;
     e = persistent_grid(kern, SH::NT, smem, tiles, &grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, SH::NT, smem, st>>>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip_flag);
-    return cudaGetLastError();
+    return launch_on(kern, dim3(grid), SH::NT, smem, st, in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip_flag);
 }
 
 template <typename T>
 cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch, int ncols,
                         const Geom& g, const FftSched& sch, const cx<T>* tw_ny, const cx<T>* tw_dct,
-                        const int* skip_flag, cudaStream_t st, int* err_bits)
+                        const int* skip_flag, LStream st, int* err_bits)
 {
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
@@ -338,9 +341,8 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
             if (err != cudaSuccess) return;
-            kern<<<grid, threads, smem, st>>>(in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
+            err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               skip_flag);
-            err = cudaGetLastError();
         };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
@@ -358,7 +360,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
 template <typename T>
 cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, long out_pitch, int ncols,
                         const Geom& g, const FftSched& sch, const cx<T>* tw_ny, const cx<T>* tw_dct,
-                        const double* dc_shift, const int* skip_flag, cudaStream_t st, int* err_bits)
+                        const double* dc_shift, const int* skip_flag, LStream st, int* err_bits)
 {
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
@@ -371,9 +373,8 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         auto go = [&](auto kern) {
             err = set_smem(kern, smem);
             if (err != cudaSuccess) return;
-            kern<<<grid, threads, smem, st>>>(in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
+            err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               dc_shift, skip_flag);
-            err = cudaGetLastError();
         };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
@@ -392,11 +393,11 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
 #if PPF_FWD
 template cudaError_t launch_yfwd<PPF_REAL>(int, const cx<PPF_REAL>*, long, cx<PPF_REAL>*, long, int, const Geom&,
                                            const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*, const int*,
-                                           cudaStream_t, int*);
+                                           LStream, int*);
 #else
 template cudaError_t launch_yinv<PPF_REAL>(int, const cx<PPF_REAL>*, long, cx<PPF_REAL>*, long, int, const Geom&,
                                            const FftSched&, const cx<PPF_REAL>*, const cx<PPF_REAL>*, const double*,
-                                           const int*, cudaStream_t, int*);
+                                           const int*, LStream, int*);
 #endif
 
 }  // namespace ppf
