@@ -55,108 +55,175 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_sum(const double* __restrict__ 
     const long i1 = min(plane, i0 + chunk);
     const double* gk = g + (long)k * plane;
     double s = 0.0;
-    for (long i = i0 + threadIdx.x; i < i1; i += blockDim.x) s += gk[i];
+#pragma unroll 8
+    for (long i = i0 + threadIdx.x; i < i1; i += ADJ_TPB) s += gk[i];
     s = block_sum(s, red);
     if (threadIdx.x == 0) colpart[(long)k * nchunk + blockIdx.x] = s;
 }
 
-// h = (g - plane mean of g) / dx3_k (dense; h may alias g)
-__global__ void __launch_bounds__(ADJ_TPB) k_adj_rhs(const double* g, double* h, const double* __restrict__ dx3,
-                                                      long plane, long chunk, int nchunk,
-                                                      const double* __restrict__ colpart)
+// sum over the chunks of level k, by one warp (valid in every lane)
+__device__ __forceinline__ double chunk_sum(const double* part, int k, int nchunk)
 {
-    __shared__ double mean;
-    const int k = blockIdx.y;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int c = 0; c < nchunk; ++c) s += colpart[(long)k * nchunk + c];
-        mean = s / (double)plane;
+    double s = 0.0;
+    for (int c = threadIdx.x & 31; c < nchunk; c += 32) s += part[(long)k * nchunk + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Zero-mode correction c(z): the transposed pinned system of the plane sums
+// (one block, sm: 4 nz doubles).  One thread's serial sweep, out of shared
+// memory so that a row costs its divide and not a round trip to L2; it runs
+// as one more block of k_adj_rhs, beside the scaling, instead of alone after
+// the solve (38 us at 128 levels).
+__device__ __forceinline__ void adj_corr(const double* __restrict__ colpart, int nchunk, int nz,
+                                         const double* __restrict__ dx3, const double* __restrict__ dmx3, double nxy,
+                                         double* __restrict__ corr, double* sm)
+{
+    double* const cs = sm;           // plane sums, then d'
+    double* const cp = sm + nz;      // c'
+    double* const am = sm + 2 * nz;  // am_k = 1/dx3_k/dmx3_k, ap_k = 1/dx3_k/dmx3_{k+1}
+    double* const ap = sm + 3 * nz;
+    for (int k = threadIdx.x >> 5; k < nz; k += ADJ_TPB / 32) {
+        const double s = chunk_sum(colpart, k, nchunk);
+        if ((threadIdx.x & 31) == 0) cs[k] = s;
+    }
+    for (int k = threadIdx.x; k < nz; k += ADJ_TPB) {
+        const double inv = __ddiv_rn(1.0, dx3[k + 1]);
+        am[k] = k == 0 ? 0.0 : __ddiv_rn(inv, dmx3[k + 1]);
+        ap[k] = k == nz - 1 ? 0.0 : __ddiv_rn(inv, dmx3[k + 2]);
     }
     __syncthreads();
-    const long i0 = (long)blockIdx.x * chunk;
+    if (threadIdx.x == 0) {
+        double tot = 0.0;
+        for (int k = 0; k < nz; ++k) tot += cs[k];
+        // zero mode of M^T g: T00^T x = cs - mean, T00^T having sub-diagonal
+        // c_{k-1} (c_0 = 0 at the pin), super-diagonal a_{k+1}, diagonal b_k (b_0 = 1);
+        // the scaled right-hand side has no zero mode, so nothing is subtracted
+        const double mean = tot / (double)nz;
+        double cprev = 0.0, dprev = 0.0;
+        for (int k = 0; k < nz; ++k) {
+            const double a = (k >= 2) ? ap[k - 1] : 0.0;
+            const double c = (k + 1 < nz) ? am[k + 1] : 0.0;
+            const double b = (k == 0) ? 1.0 : (-am[k] - ap[k]);
+            const double r = 1.0 / (b - a * cprev);
+            cprev = c * r;
+            dprev = ((cs[k] - mean) - a * dprev) * r;
+            cp[k] = cprev;
+            cs[k] = dprev;
+        }
+        for (int k = nz - 2; k >= 0; --k) cs[k] -= cp[k] * cs[k + 1];
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < nz; k += ADJ_TPB) corr[k] = cs[k] / nxy;
+}
+
+// h = (g - plane mean of g) / dx3_k (dense; h may alias g); block (0, 0) of
+// the extra column of blocks forms the zero-mode correction
+__global__ void __launch_bounds__(ADJ_TPB) k_adj_rhs(const double* g, double* h, const double* __restrict__ dx3,
+                                                      const double* __restrict__ dmx3, long plane, long chunk,
+                                                      int nchunk, const double* __restrict__ colpart,
+                                                      double* __restrict__ corr)
+{
+    extern __shared__ double adj_sm[];
+    __shared__ double mean;
+    if (blockIdx.x == 0) {
+        if (blockIdx.y == 0) adj_corr(colpart, nchunk, gridDim.y, dx3, dmx3, (double)plane, corr, adj_sm);
+        return;
+    }
+    const int k = blockIdx.y;
+    if (threadIdx.x < 32) {
+        const double s = chunk_sum(colpart, k, nchunk);
+        if (threadIdx.x == 0) mean = s / (double)plane;
+    }
+    __syncthreads();
+    const long i0 = (long)(blockIdx.x - 1) * chunk;
     const long i1 = min(plane, i0 + chunk);
     const double inv = 1.0 / dx3[k + 1], m = mean;
     const long base = (long)k * plane;
-    for (long i = i0 + threadIdx.x; i < i1; i += blockDim.x) h[base + i] = (g[base + i] - m) * inv;
-}
-
-// Zero-mode correction c(z) (one block; the serial solve runs in thread 0)
-__global__ void __launch_bounds__(ADJ_TPB) k_adj_corr(const double* __restrict__ colpart, int nchunk, int nz,
-                                                       const double* __restrict__ am, const double* __restrict__ ap,
-                                                       double nxy, double* __restrict__ corr,
-                                                       double* __restrict__ wk)
-{
-    // wk: 3 * nz doubles of scratch (plane sums, factors, solution)
-    double* cs = wk;
-    double* cp = wk + nz;
-    double* x2 = wk + 2 * nz;
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) {
-        double s = 0.0;
-        for (int c = 0; c < nchunk; ++c) s += colpart[(long)k * nchunk + c];
-        cs[k] = s;
+    // loads of several rows in flight (g and h may be the same array: each
+    // element is read before it is written, by the same thread)
+    long i = i0 + threadIdx.x;
+    for (; i + 7 * ADJ_TPB < i1; i += 8 * ADJ_TPB) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = g[base + i + q * ADJ_TPB];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) h[base + i + q * ADJ_TPB] = (v[q] - m) * inv;
     }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    double tot = 0.0;
-    for (int k = 0; k < nz; ++k) tot += cs[k];
-    // zero mode of M^T g: T00^T x = cs - mean, T00^T having sub-diagonal
-    // c_{k-1} (c_0 = 0 at the pin), super-diagonal a_{k+1}, diagonal b_k (b_0 = 1);
-    // the scaled right-hand side has no zero mode, so nothing is subtracted
-    const double mean = tot / (double)nz;
-    double cprev = 0.0, dprev = 0.0;
-    for (int k = 0; k < nz; ++k) {
-        const double a = (k >= 2) ? ap[k - 1] : 0.0;
-        const double c = (k + 1 < nz) ? am[k + 1] : 0.0;
-        const double b = (k == 0) ? 1.0 : (-am[k] - ap[k]);
-        const double r = 1.0 / (b - a * cprev);
-        cprev = c * r;
-        dprev = ((cs[k] - mean) - a * dprev) * r;
-        cp[k] = cprev;
-        x2[k] = dprev;
-    }
-    for (int k = nz - 2; k >= 0; --k) x2[k] -= cp[k] * x2[k + 1];
-    for (int k = 0; k < nz; ++k) corr[k] = x2[k] / nxy;
+    for (; i < i1; i += ADJ_TPB) h[base + i] = (g[base + i] - m) * inv;
 }
 
 // df = dx3_k * W + c_k (W: ghosted solution of the scaled right-hand side);
 // with u: per-(chunk, level) partial sums of df (u_{k-1} - u_k),
-// df (u_{k+1} - u_k), df and u.
+// df (u_{k+1} - u_k), df and u.  The row and column of an element advance by
+// the block's stride without a division (a 64-bit one per element made this
+// kernel issue-bound: 58 us at 256 x 256 x 128).
+template <bool GRAD>
 __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ W, double* __restrict__ df,
                                                       const double* __restrict__ dx3, const double* __restrict__ corr,
                                                       const double* __restrict__ u, int nx, int ny, int nz, long sy,
-                                                      long sz, long chunk, int nchunk, double* __restrict__ mpart)
+                                                      long sz, int chunk, int nchunk, double* __restrict__ mpart)
 {
     __shared__ double red[ADJ_TPB / 32];
     const int k = blockIdx.y;
-    const long plane = (long)nx * ny;
-    const long i0 = (long)blockIdx.x * chunk;
-    const long i1 = min(plane, i0 + chunk);
+    const int plane = nx * ny;
+    const int i0 = blockIdx.x * chunk, i1 = min(plane, i0 + chunk);
     const double s3 = dx3[k + 1], ck = corr[k];
+    const int dj = ADJ_TPB / nx, di = ADJ_TPB - dj * nx;
+    const double* const Wk = W + (long)(k + 1) * sz + sy + 1;
+    const double* const uk = GRAD ? u + (long)(k + 1) * sz + sy + 1 : nullptr;
+    double* const dk = df + (long)k * plane;
+    const long lo = k > 0 ? -sz : 0, hi = k < nz - 1 ? sz : 0;   // the walls' terms are zero
     double sm = 0.0, sp = 0.0, sd = 0.0, su = 0.0;
-    for (long e = i0 + threadIdx.x; e < i1; e += blockDim.x) {
-        const long j = e / nx, i = e - j * nx;
-        const long o = (i + 1) + (j + 1) * sy + (long)(k + 1) * sz;
-        const double v = s3 * W[o] + ck;
-        df[(long)k * plane + e] = v;
-        if (u) {
-            const double uc = u[o];
-            if (k > 0) sm += v * (u[o - sz] - uc);
-            if (k < nz - 1) sp += v * (u[o + sz] - uc);
+    int e = i0 + (int)threadIdx.x;
+    int j = e / nx, i = e - j * nx;
+    auto next = [&]() -> int {
+        const int o = i + j * (int)sy;
+        i += di;
+        j += dj;
+        if (i >= nx) { i -= nx; ++j; }
+        return o;
+    };
+    auto one = [&](double w, int at, double uc, double um, double up) {
+        const double v = s3 * w + ck;
+        dk[at] = v;
+        if constexpr (GRAD) {
+            sm += v * (um - uc);
+            sp += v * (up - uc);
             sd += v;
             su += uc;
         }
+    };
+    constexpr int Q = 4;   // elements in flight
+    for (; e + (Q - 1) * ADJ_TPB < i1; e += Q * ADJ_TPB) {
+        double w[Q], uc[Q], um[Q], up[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int o = next();
+            w[q] = Wk[o];
+            if constexpr (GRAD) { uc[q] = uk[o]; um[q] = uk[o + lo]; up[q] = uk[o + hi]; }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) one(w[q], e + q * ADJ_TPB, uc[q], um[q], up[q]);
     }
-    if (!u) return;
-    sm = block_sum(sm, red);
-    sp = block_sum(sp, red);
-    sd = block_sum(sd, red);
-    su = block_sum(su, red);
-    if (threadIdx.x == 0) {
-        const long q = (long)nz * nchunk, at = (long)k * nchunk + blockIdx.x;
-        mpart[at] = sm;
-        mpart[q + at] = sp;
-        mpart[2 * q + at] = sd;
-        mpart[3 * q + at] = su;
+    for (; e < i1; e += ADJ_TPB) {
+        const int o = next();
+        if constexpr (GRAD) one(Wk[o], e, uk[o], uk[o + lo], uk[o + hi]);
+        else one(Wk[o], e, 0.0, 0.0, 0.0);
+    }
+    if constexpr (GRAD) {
+        sm = block_sum(sm, red);
+        sp = block_sum(sp, red);
+        sd = block_sum(sd, red);
+        su = block_sum(su, red);
+        if (threadIdx.x == 0) {
+            const long q = (long)nz * nchunk, at = (long)k * nchunk + blockIdx.x;
+            mpart[at] = sm;
+            mpart[q + at] = sp;
+            mpart[2 * q + at] = sd;
+            mpart[3 * q + at] = su;
+        }
     }
 }
 
@@ -209,7 +276,8 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_metric(const double* __restrict
 
 int adjoint_chunks(long plane, long* chunk)
 {
-    const long target = 16384;
+    // 4096 cells a block: enough blocks and loads in flight to stream a plane
+    const long target = 4096;
     int n = (int)((plane + target - 1) / target);
     if (n < 1) n = 1;
     if (n > 64) n = 64;
@@ -219,29 +287,25 @@ int adjoint_chunks(long plane, long* chunk)
     return (int)((plane + c - 1) / c);
 }
 
-cudaError_t launch_adj_rhs(const double* g, double* h, const double* dx3, const Geom& gm, long chunk, int nchunk,
-                           double* colpart, cudaStream_t st)
+cudaError_t launch_adj_rhs(const double* g, double* h, const double* dx3, const double* dmx3, const Geom& gm,
+                           long chunk, int nchunk, double* colpart, double* corr, cudaStream_t st)
 {
     const long plane = (long)gm.nx * gm.ny;
     k_adj_sum<<<dim3(nchunk, gm.nz), ADJ_TPB, 0, st>>>(g, plane, chunk, nchunk, colpart);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_adj_rhs<<<dim3(nchunk, gm.nz), ADJ_TPB, 0, st>>>(g, h, dx3, plane, chunk, nchunk, colpart);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_adj_corr(const double* colpart, int nchunk, const Geom& gm, const double* am, const double* ap,
-                            double* corr, double* wk, cudaStream_t st)
-{
-    k_adj_corr<<<1, ADJ_TPB, 0, st>>>(colpart, nchunk, gm.nz, am, ap, (double)gm.nx * gm.ny, corr, wk);
+    // 32 KB of shared memory at the tallest column (1024 levels)
+    k_adj_rhs<<<dim3(nchunk + 1, gm.nz), ADJ_TPB, 4 * sizeof(double) * gm.nz, st>>>(g, h, dx3, dmx3, plane, chunk,
+                                                                                  nchunk, colpart, corr);
     return cudaGetLastError();
 }
 
 cudaError_t launch_adj_out(const double* W, double* df, const double* dx3, const double* corr, const double* u,
                            const Geom& gm, long chunk, int nchunk, double* mpart, cudaStream_t st)
 {
-    k_adj_out<<<dim3(nchunk, gm.nz), ADJ_TPB, 0, st>>>(W, df, dx3, corr, u, gm.nx, gm.ny, gm.nz, gm.pstride_y,
-                                                      gm.pstride_z, chunk, nchunk, mpart);
+    auto kern = u ? k_adj_out<true> : k_adj_out<false>;
+    kern<<<dim3(nchunk, gm.nz), ADJ_TPB, 0, st>>>(W, df, dx3, corr, u, gm.nx, gm.ny, gm.nz, gm.pstride_y, gm.pstride_z,
+                                                 (int)chunk, nchunk, mpart);
     return cudaGetLastError();
 }
 

@@ -610,14 +610,13 @@ int adjoint_impl(ppf_plan* p, const double* g, double* df, const double* u, doub
     double* corr = mpart + (size_t)4 * nz * nch;
     double* wk = corr + nz;
     // h = (g - plane means) / dx3 into df (aliasing g is allowed), plane sums of g
-    cudaError_t e = launch_adj_rhs(g, df, dx3, gm, p->adj_chunk, nch, colpart, st);
+    // and the zero-mode correction
+    cudaError_t e = launch_adj_rhs(g, df, dx3, dmx3, gm, p->adj_chunk, nch, colpart, corr, st);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint right-hand side");
     // W = M h with the plan's precision (refinement included); this also
     // computes the z coefficients am, ap used below
     int rc = solve_impl(p, df, p->adj_W, dmx1, dmx2, dmx3, dx3, st);
     if (rc != PPF_OK) return rc;
-    e = launch_adj_corr(colpart, nch, gm, p->am, p->ap, corr, wk, st);
-    if (e != cudaSuccess) return cuda_fail(e, "adjoint zero mode");
     e = launch_adj_out(p->adj_W, df, dx3, corr, (ddx3 || ddmx3) ? u : nullptr, gm, p->adj_chunk, nch, mpart, st);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint output");
     if (ddx3 || ddmx3) {

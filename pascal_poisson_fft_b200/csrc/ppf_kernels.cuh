@@ -205,10 +205,9 @@ cudaError_t launch_sweep_gate(const double* partials, long nblocks, double ncell
 // ---- transpose of the solve and z-metric gradient (ppf_adjoint.cu) ----
 // per-level reductions run over nchunk blocks of `chunk` cells of a plane
 int adjoint_chunks(long plane, long* chunk);
-cudaError_t launch_adj_rhs(const double* g, double* h, const double* dx3, const Geom& gm, long chunk, int nchunk,
-                           double* colpart, cudaStream_t st);
-cudaError_t launch_adj_corr(const double* colpart, int nchunk, const Geom& gm, const double* am, const double* ap,
-                            double* corr, double* wk, cudaStream_t st);
+// h = (g - plane mean) / dx3 and the zero-mode correction corr
+cudaError_t launch_adj_rhs(const double* g, double* h, const double* dx3, const double* dmx3, const Geom& gm,
+                           long chunk, int nchunk, double* colpart, double* corr, cudaStream_t st);
 cudaError_t launch_adj_out(const double* W, double* df, const double* dx3, const double* corr, const double* u,
                            const Geom& gm, long chunk, int nchunk, double* mpart, cudaStream_t st);
 cudaError_t launch_adj_metric(const double* mpart, int nchunk, const Geom& gm, const double* am, const double* ap,
