@@ -34,7 +34,7 @@ namespace ppf {
 // z solve beside the transform tiles.  Its own entry point: the call costs
 // the large transforms registers (512^3 mixed solve +1 % with it in k_xfwd).
 template <typename T, bool DCT, typename SH>
-__global__ void __launch_bounds__(512, (SH::CT && SH::NT <= 256) ? 2 : 0)
+__global__ void __launch_bounds__(512, (!SH::CT || SH::NT <= 256) ? 2 : 0)
     k_xfwd_prep(PPF_XFWD_PARAMS, const __grid_constant__ ZPrep zp, unsigned nprep)
 {
     pdl_enter();
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(512, (SH::CT && SH::NT <= 256) ? 2 : 0)
 // the plain periodic transform of 384-point tiles (768-point lines) is bounded
 // to four resident CTAs of 384 threads: 32 registers, five CTAs fit an SM
 template <typename T, bool DCT, int RESID, typename SH>
-__global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 : 0) k_xfwd(PPF_XFWD_PARAMS)
+__global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 : (!SH::CT && RESID == 0) ? 2 : 0) k_xfwd(PPF_XFWD_PARAMS)
 {
     pdl_enter();
     xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PA
     (long)blockIdx.x
 
 template <typename T, bool DCT, bool ACC, bool GHOST, typename SH, int UK = U_P>
-__global__ void __launch_bounds__(512) k_xinv(PPF_XINV_PARAMS)
+__global__ void __launch_bounds__(512, SH::CT ? 0 : 2) k_xinv(PPF_XINV_PARAMS)
 {
     pdl_enter();
     xinv<T, DCT, ACC, GHOST, SH, UK>(PPF_XINV_ARGS);

@@ -124,6 +124,8 @@ __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn
     const double* const f0 = f + line0 * nx;   // the tile's lines are contiguous: pair (l, n) at 2 e
     T* const sr = reinterpret_cast<T*>(s);
 
+    // run-time tiles: eight elements a thread at most, the loads of four issued together
+#pragma unroll (CT || RESID ? 1 : 4)
     for (int e = threadIdx.x; e < E; e += NTH) {
         const int l = div_n<SH>(e, sch), n = e - l * nc;
         double a = 0.0, b = 0.0;
@@ -284,6 +286,7 @@ __device__ __forceinline__ void xinv(const void* __restrict__ in_, long in_pitch
     // Z_{nc-k} from (X_{nc-k}, conj X_k).  DCT: X_j = e^{i pi j/(2 nx)} (C_j -
     // i C_{nx-j}) of the coefficients C (cuda_Poisson_DCT_b_pre), C_nx = 0.
     const int NP = nc / 2 + 1;
+#pragma unroll (CT || (sizeof(T) == 4 && ACC) ? 1 : 2)
     for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
         const int l = div_np<SH>(e, sch), k = e - l * NP;
         const int kc = nc - k;

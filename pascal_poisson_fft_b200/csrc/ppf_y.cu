@@ -41,8 +41,10 @@ struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
 
 // resident CTAs asked of the compile-time y tiles of the DCT and packed-real
 // kinds
+// (run-time tiles: 64 registers at the largest block, so that three 320-thread
+// blocks of a 320-point FP64 tile fit an SM instead of two)
 template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
-template <typename SH> constexpr int y_ctas = !SH::CT ? 0 : SH::NT <= 256 ? 4 : 2;
+template <typename SH> constexpr int y_ctas = SH::CT && SH::NT <= 256 ? 4 : 2;
 
 template <typename T, int KIND, typename SH>
 __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,

@@ -37,6 +37,8 @@ __device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch
     const int ip = (int)in_pitch, op = (int)out_pitch;
     const int E = ny << lgW;
 
+    // run-time tiles: eight elements a thread at most, the loads of four issued together
+#pragma unroll (CT ? 1 : 4)
     for (int e = threadIdx.x; e < E; e += NTH) {
         const int l = e & (W - 1), y = e >> lgW;
         cx<T> v = mk<T>((T)0, (T)0);
@@ -112,6 +114,7 @@ __device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch
     const int ip = (int)in_pitch, op = (int)out_pitch;
     if (KIND == Y_C2C) {
         const cx<T>* inp = in + (long)z * ny * in_pitch + col0;
+#pragma unroll (CT ? 1 : 4)
         for (int e = threadIdx.x; e < E; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
             cx<T> v = mk<T>((T)0, (T)0);
@@ -126,6 +129,7 @@ __device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch
         // i X_{n-k}), Z_{n-k} = w (X_k + i X_{n-k}) from one read of the pair
         const cx<T>* inp = in + (long)z * ny * in_pitch + col0;
         const int Eh = (ny / 2 + 1) << lgW;
+#pragma unroll (CT ? 1 : 2)
         for (int e = threadIdx.x; e < Eh; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
             cx<T> Z = mk<T>((T)0, (T)0), Zp = Z;
@@ -146,6 +150,7 @@ __device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch
         const int my = ny / 2 + 1;
         const cx<T>* inp = in + (long)z * my * in_pitch + 2 * col0;
         const int Eh = my << lgW;
+#pragma unroll (CT ? 1 : 2)
         for (int e = threadIdx.x; e < Eh; e += NTH) {
             const int l = e & (W - 1), k = e >> lgW;
             cx<T> Z = mk<T>((T)0, (T)0), Zp = Z;
