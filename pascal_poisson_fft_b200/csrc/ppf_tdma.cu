@@ -1664,10 +1664,244 @@ __global__ void __launch_bounds__(TPB) k_thomas_cycl(const double* __restrict__ 
     }
 }
 
+// tdma_many with its factors kept on chip: one warp per block, a system per
+// lane.  c' of every row stays in shared memory and d' goes to d in place (or
+// to shared memory, KEEPD), so every row of a, b, c, d is read once and the
+// back substitution is one multiply and one subtract a row: k_thomas_arr
+// reads the arrays twice and runs the reciprocal chain twice.  The next
+// chunk's rows load while the current one is eliminated.  The same operations
+// in the same order: the same bits.
+constexpr int SYS_C = 8;    // rows per chunk, elimination
+constexpr int SYS_B = 16;   // substitution
+
+template <bool KEEPD>
+__global__ void __launch_bounds__(32) k_thomas_sys(const double* __restrict__ a, const double* __restrict__ b,
+                                                   const double* __restrict__ c, double* d, int n_sys, int n)
+{
+    extern __shared__ double sys_sm[];
+    constexpr int C = SYS_C;
+    const long sys = (long)blockIdx.x * 32 + threadIdx.x;
+    if (sys >= n_sys) return;
+    double* const cs = sys_sm + threadIdx.x;                    // c', [n][32]
+    double* const ds = sys_sm + (size_t)n * 32 + threadIdx.x;   // KEEPD: d'
+    const double *pa = a + sys, *pb = b + sys, *pc = c + sys;
+    double* const pd = d + sys;
+    double av[2][C], bv[2][C], cv[2][C], dv[2][C];
+    auto load = [&](int z0, double* A, double* B, double* Cc, double* Dd) {
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            A[q] = 0.0; B[q] = 1.0; Cc[q] = 0.0; Dd[q] = 0.0;
+            if (z0 + q < n) {
+                const long o = (long)(z0 + q) * n_sys;
+                A[q] = __ldg(pa + o); B[q] = __ldg(pb + o); Cc[q] = __ldg(pc + o); Dd[q] = pd[o];
+            }
+        }
+    };
+    double cp = 0.0, dp = 0.0;
+    auto elim = [&](int z0, const double* A, const double* B, const double* Cc, const double* Dd) {
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const int z = z0 + q;
+            if (z < n) {
+                if (q == 0 && z0 == 0) {
+                    dp = __ddiv_rn(Dd[0], B[0]);
+                    cp = __ddiv_rn(Cc[0], B[0]);
+                } else {
+                    const double t = __dsub_rn(Dd[q], __dmul_rn(A[q], dp));
+                    const double r = __drcp_rn(__dsub_rn(B[q], __dmul_rn(A[q], cp)));
+                    cp = __dmul_rn(r, Cc[q]);
+                    dp = __dmul_rn(r, t);
+                }
+                cs[z * 32] = cp;
+                if constexpr (KEEPD) ds[z * 32] = dp;
+                else pd[(long)z * n_sys] = dp;
+            }
+        }
+    };
+    load(0, av[0], bv[0], cv[0], dv[0]);
+    for (int z0 = 0; z0 < n; z0 += 2 * C) {
+        load(z0 + C, av[1], bv[1], cv[1], dv[1]);
+        elim(z0, av[0], bv[0], cv[0], dv[0]);
+        load(z0 + 2 * C, av[0], bv[0], cv[0], dv[0]);
+        elim(z0 + C, av[1], bv[1], cv[1], dv[1]);
+    }
+    double x = dp;
+    pd[(long)(n - 1) * n_sys] = x;
+    constexpr int B2 = SYS_B;
+    double v[2][B2];
+    // rows z1, z1 - 1, ..: d' of the next chunk loads ahead
+    auto loadd = [&](int z1, double* V) {
+        if constexpr (!KEEPD) {
+#pragma unroll
+            for (int q = 0; q < B2; ++q) V[q] = z1 - q >= 0 ? pd[(long)(z1 - q) * n_sys] : 0.0;
+        }
+    };
+    auto subst = [&](int z1, const double* V) {
+#pragma unroll
+        for (int q = 0; q < B2; ++q) {
+            const int z = z1 - q;
+            if (z >= 0) {
+                const double dq = KEEPD ? ds[z * 32] : V[q];
+                x = __dsub_rn(dq, __dmul_rn(cs[z * 32], x));
+                pd[(long)z * n_sys] = x;
+            }
+        }
+    };
+    loadd(n - 2, v[0]);
+    for (int z1 = n - 2; z1 >= 0; z1 -= 2 * B2) {
+        loadd(z1 - B2, v[1]);
+        subst(z1, v[0]);
+        loadd(z1 - 2 * B2, v[0]);
+        subst(z1 - B2, v[1]);
+    }
+}
+
+// The cyclic sequence the same way: c' and e' of rows 1 .. n-1 in shared
+// memory, d' in place; the first back substitution leaves y in place and e in
+// shared memory, the second is x_i = y_i + x_0 e_i of independent rows.
+__global__ void __launch_bounds__(32) k_thomas_sys_cycl(const double* __restrict__ a, const double* __restrict__ b,
+                                                        const double* __restrict__ c, double* d, int n_sys, int n)
+{
+    extern __shared__ double sys_sm[];
+    constexpr int C = SYS_C;
+    const long sys = (long)blockIdx.x * 32 + threadIdx.x;
+    if (sys >= n_sys) return;
+    double* const cs = sys_sm + threadIdx.x;                    // c', [n][32]
+    double* const es = sys_sm + (size_t)n * 32 + threadIdx.x;   // e', then e
+    const double *pa = a + sys, *pb = b + sys, *pc = c + sys;
+    double* const pd = d + sys;
+    const double e_first = -__ldg(pa + n_sys), e_last = -__ldg(pc + (long)(n - 1) * n_sys);
+    double av[2][C], bv[2][C], cv[2][C], dv[2][C];
+    auto load = [&](int z0, double* A, double* B, double* Cc, double* Dd) {
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            A[q] = 0.0; B[q] = 1.0; Cc[q] = 0.0; Dd[q] = 0.0;
+            if (z0 + q < n) {
+                const long o = (long)(z0 + q) * n_sys;
+                A[q] = __ldg(pa + o); B[q] = __ldg(pb + o); Cc[q] = __ldg(pc + o); Dd[q] = pd[o];
+            }
+        }
+    };
+    double cp = 0.0, dp = 0.0, ep = 0.0;
+    auto elim = [&](int z0, const double* A, const double* B, const double* Cc, const double* Dd) {
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const int z = z0 + q;
+            if (z < n) {
+                // e(2) = -a(2) is set before e(n) = -c(n)
+                const double ei = z == n - 1 ? e_last : (z == 1 ? e_first : 0.0);
+                if (q == 0 && z0 == 1) {
+                    dp = __ddiv_rn(Dd[0], B[0]);
+                    ep = __ddiv_rn(ei, B[0]);
+                    cp = __ddiv_rn(Cc[0], B[0]);
+                } else {
+                    const double t = __dsub_rn(Dd[q], __dmul_rn(A[q], dp));
+                    const double u = __dsub_rn(ei, __dmul_rn(A[q], ep));
+                    const double r = __drcp_rn(__dsub_rn(B[q], __dmul_rn(A[q], cp)));
+                    cp = __dmul_rn(r, Cc[q]);
+                    dp = __dmul_rn(r, t);
+                    ep = __dmul_rn(r, u);
+                }
+                cs[z * 32] = cp;
+                es[z * 32] = ep;
+                pd[(long)z * n_sys] = dp;
+            }
+        }
+    };
+    load(1, av[0], bv[0], cv[0], dv[0]);
+    for (int z0 = 1; z0 < n; z0 += 2 * C) {
+        load(z0 + C, av[1], bv[1], cv[1], dv[1]);
+        elim(z0, av[0], bv[0], cv[0], dv[0]);
+        load(z0 + 2 * C, av[0], bv[0], cv[0], dv[0]);
+        elim(z0 + C, av[1], bv[1], cv[1], dv[1]);
+    }
+    const double d_top = dp, e_top = ep;
+    double y = dp, e = ep;
+    constexpr int B2 = SYS_B;
+    double v[2][B2];
+    auto loadd = [&](int z1, double* V) {
+#pragma unroll
+        for (int q = 0; q < B2; ++q) V[q] = z1 - q >= 1 ? pd[(long)(z1 - q) * n_sys] : 0.0;
+    };
+    auto subst = [&](int z1, const double* V) {
+#pragma unroll
+        for (int q = 0; q < B2; ++q) {
+            const int z = z1 - q;
+            if (z >= 1) {
+                const double cq = cs[z * 32];
+                y = __dsub_rn(V[q], __dmul_rn(cq, y));
+                e = __dsub_rn(es[z * 32], __dmul_rn(cq, e));
+                es[z * 32] = e;
+                pd[(long)z * n_sys] = y;
+            }
+        }
+    };
+    loadd(n - 2, v[0]);
+    for (int z1 = n - 2; z1 >= 1; z1 -= 2 * B2) {
+        loadd(z1 - B2, v[1]);
+        subst(z1, v[0]);
+        loadd(z1 - 2 * B2, v[0]);
+        subst(z1 - B2, v[1]);
+    }
+    // d(1) = (d(1) - a(1) d(n) - c(1) d(2)) / (b(1) + a(1) e(n) + c(1) e(2))
+    const double a0 = __ldg(pa), b0 = __ldg(pb), c0 = __ldg(pc);
+    const double x0 = __ddiv_rn(__dsub_rn(__dsub_rn(pd[0], __dmul_rn(a0, d_top)), __dmul_rn(c0, y)),
+                                __dadd_rn(__dadd_rn(b0, __dmul_rn(a0, e_top)), __dmul_rn(c0, e)));
+    pd[0] = x0;
+    for (int z0 = 1; z0 < n; z0 += B2) {
+        double w[B2];
+#pragma unroll
+        for (int q = 0; q < B2; ++q) w[q] = z0 + q < n ? pd[(long)(z0 + q) * n_sys] : 0.0;
+#pragma unroll
+        for (int q = 0; q < B2; ++q)
+            if (z0 + q < n) pd[(long)(z0 + q) * n_sys] = __dadd_rn(w[q], __dmul_rn(x0, es[(z0 + q) * 32]));
+    }
+}
+
+// The on-chip kernels where they are faster: every block resident at once
+// (four a SM at most unless cyclic), where the chains are the time; or many
+// short columns (cyclic: four blocks a SM), where one read instead of two (three) is.
+// In between one wave after another of chains costs more than the reads saved.
+// Measured, k_thomas_arr / k_thomas_cycl -> these (systems x rows): 5922 x 118
+// 37 -> 25 us, 20000 x 64 24 -> 16, 4000 x 440 117 -> 72, 300000 x 32 91 -> 72,
+// but 42206 x 70 30 -> 34, 65536 x 256 236 -> 289; cyclic 4000 x 440 201 ->
+// 95, 300000 x 100 541 -> 474, 131072 x 128 (three a SM) 329 = 326.  Under 24
+// rows the launch is all there is (1000 x 16 14.0 -> 14.9).
+cudaError_t launch_tdma_sys(const double* a, const double* b, const double* c, double* d, int n_sys, int n_row,
+                            bool cyclic, cudaStream_t st, bool* used)
+{
+    *used = false;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const long blocks = ((long)n_sys + 31) / 32;
+    const size_t one = (size_t)n_row * 32 * sizeof(double);
+    auto resident = [&](size_t smem) { return smem > 226 * 1024 ? 0L : std::min(32L, (long)(227 * 1024 / (smem + 1024))); };
+    const bool keepd = !cyclic && resident(2 * one) * sms >= blocks;
+    const size_t smem = (cyclic || keepd ? 2 : 1) * one;
+    const long per = resident(smem);
+    const bool few = blocks <= per * sms && (cyclic || blocks <= 4L * sms);
+    const bool many = per >= (cyclic ? 4 : 6) && (cyclic || n_row <= 40);
+    if (n_row < 24 || !(few || many)) return cudaSuccess;
+    auto go = [&](auto kern) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<(unsigned)blocks, 32, smem, st>>>(a, b, c, d, n_sys, n_row);
+        return cudaGetLastError();
+    };
+    *used = true;
+    if (cyclic) return go(k_thomas_sys_cycl);
+    return keepd ? go(k_thomas_sys<true>) : go(k_thomas_sys<false>);
+}
+
 cudaError_t launch_tdma_many(const double* a, const double* b, const double* c, double* d, int n_sys, int n_row,
                              bool cyclic, int* err, cudaStream_t st)
 {
     (void)err;
+    bool used = false;
+    const cudaError_t se = launch_tdma_sys(a, b, c, d, n_sys, n_row, cyclic, st, &used);
+    if (used || se != cudaSuccess) return se;
     const int m = cyclic ? n_row - 1 : n_row;
     const int nch = (m + CH - 1) / CH;
     const size_t smem = (size_t)(cyclic ? 3 : 2) * nch * TPB * sizeof(double);
