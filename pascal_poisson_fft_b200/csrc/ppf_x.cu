@@ -30,11 +30,16 @@ namespace ppf {
         const cx<T>* __restrict__ tw_dct, const int* __restrict__ skip
 #define PPF_XFWD_ARGS(tile) f, rs, g, out_, out_pitch, sch, Wrt, lgWrt, tw_half, tw_n, tw_dct, skip, tile
 
+// FP64 compile-time tiles: resident CTAs per SM asked of the compiler.  Five
+// of 256 threads (48 registers); of 384 threads two (80): the five once asked
+// left 32 registers and 0.5 to 1 KB of spills a thread.
+constexpr int x64_ctas(int threads) { return threads > 256 ? 2 : 1280 / threads; }
+
 // The x forward of a solve with z tables: the first nprep blocks prepare the
 // z solve beside the transform tiles.  Its own entry point: the call costs
 // the large transforms registers (512^3 mixed solve +1 % with it in k_xfwd).
 template <typename T, bool DCT, typename SH>
-__global__ void __launch_bounds__(512, (!SH::CT || SH::NT <= 256) ? 2 : 0)
+__global__ void __launch_bounds__(SH::CT ? SH::NT : 512, SH::CT && sizeof(T) == 8 ? x64_ctas(SH::NT) : (!SH::CT || SH::NT <= 256) ? 2 : 0)
     k_xfwd_prep(PPF_XFWD_PARAMS, const __grid_constant__ ZPrep zp, unsigned nprep)
 {
     pdl_enter();
@@ -55,10 +60,6 @@ __global__ void __launch_bounds__(512, (SH::N == 384 && !DCT && RESID == 0) ? 4 
     xfwd<T, DCT, RESID, SH>(PPF_XFWD_ARGS((long)blockIdx.x));
 }
 
-// FP64 compile-time tiles: resident CTAs per SM asked of the compiler.  Five
-// of 256 threads (48 registers); of 384 threads two (80): the five once asked
-// left 32 registers and 0.5 to 1 KB of spills a thread.
-constexpr int x64_ctas(int threads) { return threads > 256 ? 2 : 5; }
 template <bool DCT, typename SH, typename T = double>
 __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PARAMS)
 {

@@ -286,7 +286,8 @@ __device__ __forceinline__ void xinv(const void* __restrict__ in_, long in_pitch
     // Z_{nc-k} from (X_{nc-k}, conj X_k).  DCT: X_j = e^{i pi j/(2 nx)} (C_j -
     // i C_{nx-j}) of the coefficients C (cuda_Poisson_DCT_b_pre), C_nx = 0.
     const int NP = nc / 2 + 1;
-#pragma unroll (CT || (sizeof(T) == 4 && ACC) ? 1 : 2)
+    // (FP64 compile-time tiles by four: 512^3 x inverse 516 -> 499 us)
+#pragma unroll (CT ? (sizeof(T) == 8 ? 4 : 1) : (sizeof(T) == 4 && ACC) ? 1 : 2)
     for (int e = threadIdx.x; e < (NP << lgW); e += NTH) {
         const int l = div_np<SH>(e, sch), k = e - l * NP;
         const int kc = nc - k;

@@ -44,11 +44,17 @@ inline int pick_w(int n, int& threads)
     return W;
 }
 
-// Compile-time shapes of the common lengths: W lines, NT threads (16 FP32
-// or 8 FP64 elements per thread), radix sequence.  Other lengths use the
-// run-time engine.  XINV: the shape of the x inverse, whose FP32 384-point
-// lines run faster with the radix-3 pass last (the other transforms with it
-// first); the tile width is the same either way.
+// Compile-time shapes of the common lengths: W lines, NT threads (8 elements
+// a thread, 16 in the FP32 32- and 512-point tiles), radix sequence.  Other
+// lengths use the run-time engine.  The short lines' tiles are kept small (16
+// lines of 64 points, 8 FP64 or 16 FP32 lines of 128) so that small grids
+// have tiles for every SM and enough resident; FP32 tiles of 16 columns also
+// take the paired, TMA-fed y pipeline.  Against 64 lines of 64 and 32 of 128
+// points: mixed 128^3 (one sweep, with stage events) 200 -> 187 us, 128 x 256
+// x 200 388 -> 375; FP64 128^3 91 -> 87, 256^3 394 -> 386.  XINV: the shape of
+// the x inverse, whose FP32 384-point lines run faster with the radix-3 pass
+// last (the other transforms with it first); the tile width is the same
+// either way.
 template <typename T, bool XINV = false, typename F>
 void with_shape(const FftSched& sch, F&& f)
 {
@@ -56,9 +62,9 @@ void with_shape(const FftSched& sch, F&& f)
     if (sch.rt) { f(ShapeRT{}); return; }
     if constexpr (sizeof(T) == 8) {
         switch (n) {
-            case 32:  f(ShapeCT<32, 64, 256, 8, 4>{}); return;
-            case 64:  f(ShapeCT<64, 32, 256, 8, 8>{}); return;
-            case 128: f(ShapeCT<128, 16, 256, 8, 4, 4>{}); return;
+            case 32:  f(ShapeCT<32, 32, 128, 8, 4>{}); return;
+            case 64:  f(ShapeCT<64, 16, 128, 8, 8>{}); return;
+            case 128: f(ShapeCT<128, 8, 128, 8, 4, 4>{}); return;
             case 256: f(ShapeCT<256, 8, 256, 8, 8, 4>{}); return;
             case 384: f(ShapeCT<384, 8, 384, 8, 4, 4, 3>{}); return;
             case 512: f(ShapeCT<512, 8, 512, 8, 8, 8>{}); return;
@@ -68,8 +74,8 @@ void with_shape(const FftSched& sch, F&& f)
     } else {
         switch (n) {
             case 32:  f(ShapeCT<32, 128, 256, 8, 4>{}); return;
-            case 64:  f(ShapeCT<64, 64, 256, 8, 8>{}); return;
-            case 128: f(ShapeCT<128, 32, 256, 8, 4, 4>{}); return;
+            case 64:  f(ShapeCT<64, 16, 128, 8, 8>{}); return;
+            case 128: f(ShapeCT<128, 16, 256, 8, 4, 4>{}); return;
             case 256: f(ShapeCT<256, 8, 256, 8, 8, 4>{}); return;
             case 384:
                 if constexpr (XINV) f(ShapeCT<384, 8, 384, 8, 4, 4, 3>{});

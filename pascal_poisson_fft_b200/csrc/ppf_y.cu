@@ -44,7 +44,7 @@ struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
 // (run-time tiles: 64 registers at the largest block, so that three 320-thread
 // blocks of a 320-point FP64 tile fit an SM instead of two)
 template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
-template <typename SH> constexpr int y_ctas = SH::CT && SH::NT <= 256 ? 4 : 2;
+template <typename SH> constexpr int y_ctas = SH::CT && SH::NT <= 256 ? 1024 / SH::NT : 2;
 
 template <typename T, int KIND, typename SH>
 __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* __restrict__
 // bounds the registers to 85 a thread; two of the 384-thread shapes (three
 // left 56 registers and 200 bytes of spills)
 template <bool INV, typename SH>
-__global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 3) k_y_c2c_pipe64(const cx<double>* __restrict__ in, long in_pitch,
+__global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 768 / SH::NT) k_y_c2c_pipe64(const cx<double>* __restrict__ in, long in_pitch,
                                                            cx<double>* __restrict__ out, long out_pitch, int ncols,
                                                            int nz, const cx<double>* __restrict__ tw,
                                                            const double* __restrict__ dc_shift,
