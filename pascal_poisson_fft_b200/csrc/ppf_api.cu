@@ -59,46 +59,42 @@ void cexp_tab(int count, long double num, long double den, std::vector<double>& 
 }
 
 // The fewest passes, then the largest smallest radix, of a descending radix
-// sequence of n; false if n has a factor other than 2, 3, 5.
-bool few_passes(int n, int top, size_t elem, std::vector<int>& cur, std::vector<int>& best)
+// sequence of n (of factors 2, 3, 5 only).
+void few_passes(int n, int top, std::vector<int>& cur, std::vector<int>& best)
 {
     if (n == 1) {
         if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && cur.back() > best.back()))
             best = cur;
-        return true;
+        return;
     }
-    if (!best.empty() && cur.size() + 1 > best.size()) return true;
-    bool any = false;
-    for (int r : { 10, 9, 8, 6, 5, 4, 3, 2 }) {
-        if (r > top || n % r || (elem == 8 && (r == 6 || r > 8))) continue;
+    if (!best.empty() && cur.size() + 1 > best.size()) return;
+    for (int r : { 8, 5, 4, 3, 2 }) {
+        if (r > top || n % r) continue;
         cur.push_back(r);
-        any |= few_passes(n / r, r, elem, cur, best);
+        few_passes(n / r, r, cur, best);
         cur.pop_back();
     }
-    return any;
 }
 
 // Radix schedule of a length-n transform of FP64 (elem 8) or FP32 (4) data.
-// order 0: the fewest passes (FP64 of radices 2, 3, 4, 5, 8; FP32 also 6, 9,
-// 10; every pass is one round trip of the tile through shared
-// memory and a barrier: 90 = 10 9, 360 = 10 6 6, 720 = 10 9 8, where radices
-// 2, 3, 4, 5, 8 need 4, 5 and 5); 1: radices 4, 2, 3, 5; 2: radices 3 and 5
-// first, then 8, 4, 2.
+// order 0: FP64, the fewest passes of radices 8, 5, 4, 3, 2 (every pass is one
+// round trip of the tile through shared memory and a barrier; radices 6, 9
+// and 10 would save more passes but take 103 to 120 registers against 70, y of
+// 576 points 85 -> 116 us); FP32, radix 8 first, then 4, 2, 3, 5, whose
+// results stay as they are to the bit.  1: radices 4, 2, 3, 5; 2: radices 3
+// and 5 first, then 8, 4, 2.
 bool factor(int n, FftSched& s, size_t elem, int order_id = 0)
 {
-    static const int orders[3][5] = { { 0, 0, 0, 0, 0 }, { 4, 2, 3, 5, 0 }, { 3, 5, 8, 4, 2 } };
+    static const int orders[3][5] = { { 8, 4, 2, 3, 5 }, { 4, 2, 3, 5, 0 }, { 3, 5, 8, 4, 2 } };
     s = FftSched{};
     s.n = n;
     if (n < 1 || order_id < 0 || order_id > 2) return false;
     int m = n;
-    if (order_id == 0) {
+    if (order_id == 0 && elem == 8) {
+        for (int r : { 2, 3, 5 })
+            while (m % r == 0) m /= r;
         std::vector<int> cur, best;
-        if (n > 1) {
-            for (int r : { 2, 3, 5 })
-                while (m % r == 0) m /= r;
-            if (m != 1) return false;
-            few_passes(n, 10, elem, cur, best);
-        }
+        if (n > 1 && m == 1) few_passes(n, 8, cur, best);
         if (best.size() > 12) return false;
         for (int r : best) s.radix[s.npass++] = r;
     } else {
@@ -300,6 +296,9 @@ long plan_ztab(const ppf_plan* p)
     if (!f32 && pair && !p->g.pz) mb = 512;
     if (f32 && !p->cplx) mb = 32;
     const long cells = (long)p->g.nx * p->g.ny * p->g.nz;
+    // where the streamed FP32 bulk would run its twisted sweep (a block of 256
+    // values for every SM), whose roundings the tables' sweep does not share
+    if (f32 && p->b_pitch * (long)p->my * (p->cplx ? 2 : 1) >= 147L * 256) return 0;
     if (f32 && p->g.nz > 160 && cells < 5000000 && p->b_pitch * (long)p->my > 4096) return 0;
     if (field > (mb << 20)) return 0;
     return ztab_doubles(p->g.nz, p->b_pitch * (long)ztab_rows(p), p->g.pz, f32);

@@ -25,9 +25,6 @@ template <> struct K<double> {
     static constexpr double s2 = 0.58778525229247312917;   // sin(4pi/5)
     static constexpr double c16 = 0.92387953251128675613;  // cos(pi/8)
     static constexpr double s16 = 0.38268343236508977173;  // sin(pi/8)
-    static constexpr double c9a = 0.76604444311897803520, s9a = 0.64278760968653932632;   // cos, sin(2pi/9)
-    static constexpr double c9b = 0.17364817766693034885, s9b = 0.98480775301220805937;   // cos, sin(4pi/9)
-    static constexpr double c9d = -0.93969262078590838405, s9d = 0.34202014332566873304;  // cos, sin(8pi/9)
 };
 template <> struct K<float> {
     static constexpr float s3 = 0.86602540378443864676f;
@@ -38,9 +35,6 @@ template <> struct K<float> {
     static constexpr float s2 = 0.58778525229247312917f;
     static constexpr float c16 = 0.92387953251128675613f;
     static constexpr float s16 = 0.38268343236508977173f;
-    static constexpr float c9a = 0.76604444311897803520f, s9a = 0.64278760968653932632f;
-    static constexpr float c9b = 0.17364817766693034885f, s9b = 0.98480775301220805937f;
-    static constexpr float c9d = -0.93969262078590838405f, s9d = 0.34202014332566873304f;
 };
 
 template <typename T, bool INV, int R> struct Dft;
@@ -161,107 +155,21 @@ template <typename T, bool INV> struct Dft<T, INV, 16> {
     }
 };
 
-// x (c - i s) forward, x (c + i s) inverse
-template <typename T, bool INV>
-__device__ __forceinline__ cx<T> rot(cx<T> x, T c, T s)
-{
-    return cmul(x, mk(c, INV ? s : -s));
-}
-
-// Composite radices of the run-time engine: 2 x 3, 3 x 3 and 2 x 5
-template <typename T, bool INV> struct Dft<T, INV, 6> {
-    static __device__ __forceinline__ void run(cx<T>* v)
-    {
-        cx<T> a[3], b[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            a[k] = v[k] + v[k + 3];
-            b[k] = v[k] - v[k + 3];
-        }
-        b[1] = rot<T, INV>(b[1], (T)0.5, K<T>::s3);
-        b[2] = rot<T, INV>(b[2], (T)-0.5, K<T>::s3);
-        Dft<T, INV, 3>::run(a);
-        Dft<T, INV, 3>::run(b);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            v[2 * m] = a[m];
-            v[2 * m + 1] = b[m];
-        }
-    }
-};
-
-template <typename T, bool INV> struct Dft<T, INV, 9> {
-    static __device__ __forceinline__ void run(cx<T>* v)
-    {
-        cx<T> t[3][3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) t[k][j] = v[k + 3 * j];
-            Dft<T, INV, 3>::run(t[k]);
-        }
-        t[1][1] = rot<T, INV>(t[1][1], K<T>::c9a, K<T>::s9a);
-        t[1][2] = rot<T, INV>(t[1][2], K<T>::c9b, K<T>::s9b);
-        t[2][1] = rot<T, INV>(t[2][1], K<T>::c9b, K<T>::s9b);
-        t[2][2] = rot<T, INV>(t[2][2], K<T>::c9d, K<T>::s9d);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            cx<T> u[3] = { t[0][j], t[1][j], t[2][j] };
-            Dft<T, INV, 3>::run(u);
-            v[j] = u[0];
-            v[j + 3] = u[1];
-            v[j + 6] = u[2];
-        }
-    }
-};
-
-template <typename T, bool INV> struct Dft<T, INV, 10> {
-    static __device__ __forceinline__ void run(cx<T>* v)
-    {
-        cx<T> a[5], b[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            a[k] = v[k] + v[k + 5];
-            b[k] = v[k] - v[k + 5];
-        }
-        // e^{-i pi k/5}: cos 36 = -c2, cos 72 = c1, sin 36 = s2, sin 72 = s1
-        b[1] = rot<T, INV>(b[1], -K<T>::c2, K<T>::s2);
-        b[2] = rot<T, INV>(b[2], K<T>::c1, K<T>::s1);
-        b[3] = rot<T, INV>(b[3], -K<T>::c1, K<T>::s1);
-        b[4] = rot<T, INV>(b[4], K<T>::c2, K<T>::s2);
-        Dft<T, INV, 5>::run(a);
-        Dft<T, INV, 5>::run(b);
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            v[2 * m] = a[m];
-            v[2 * m + 1] = b[m];
-        }
-    }
-};
-
 // The twiddles w^r (r = 1..R-1, w = tw[k ts]) of one butterfly applied to
 // its inputs v[1..R-1].  FP64 reads every power from the table.  FP32 reads
 // w and forms w^2 = w w, w^3 = w w^2, w^4 = w^2 w^2, w^5 = w^4 w,
 // w^6 = w^4 w^2, w^7 = w^4 w^3 (at most three products deep, a few ulp of
 // FP32, which the FP64 refinement absorbs): one load instead of R-1 in the
-// passes the FP32 y kernels are bound by.  Radices 9 and 10 also read w^5
-// and form w^6..w^9 from it, so no power is deeper.
+// passes the FP32 y kernels are bound by.
 template <typename T, bool INV, int R>
 __device__ __forceinline__ void twiddle_powers(cx<T>* w, const cx<T>* __restrict__ tw, int k, int ts)
 {
-    static_assert(sizeof(T) == 4 && (R == 4 || R == 5 || R == 6 || R >= 8), "FP32 radix 4, 5, 6, 8, 9 or 10");
+    static_assert(sizeof(T) == 4 && (R == 4 || R == 5 || R == 8), "FP32 radix 4, 5 or 8");
     w[1] = ldg(tw + k * ts);
     if (INV) w[1].y = -w[1].y;
     w[2] = cmul(w[1], w[1]);
     w[3] = cmul(w[1], w[2]);
     if constexpr (R >= 5) w[4] = cmul(w[2], w[2]);
-    if constexpr (R == 6) w[5] = cmul(w[4], w[1]);
-    if constexpr (R >= 9) {
-        w[5] = ldg(tw + 5 * k * ts);
-        if (INV) w[5].y = -w[5].y;
-#pragma unroll
-        for (int r = 6; r < R; ++r) w[r] = cmul(w[5], w[r - 5]);
-    }
     if constexpr (R == 8) {
         w[5] = cmul(w[4], w[1]);
         w[6] = cmul(w[4], w[2]);
@@ -272,7 +180,7 @@ __device__ __forceinline__ void twiddle_powers(cx<T>* w, const cx<T>* __restrict
 template <typename T, bool INV, int R>
 __device__ __forceinline__ void twiddle_mul(cx<T>* v, const cx<T>* __restrict__ tw, int k, int ts)
 {
-    if constexpr (sizeof(T) == 4 && (R == 4 || R == 5 || R == 6 || R >= 8)) {
+    if constexpr (sizeof(T) == 4 && (R == 4 || R == 5 || R == 8)) {
         cx<T> w[R];
         twiddle_powers<T, INV, R>(w, tw, k, ts);
 #pragma unroll
@@ -294,16 +202,16 @@ __device__ __forceinline__ void twiddle_mul(cx<T>* v, const cx<T>* __restrict__ 
 // tw[k] = e^{-2 pi i k/n}; mg: fast_div multiplier of Ns.  v is the caller's
 // register buffer (VMAX complex), shared by every radix so that all passes
 // reuse the same registers.
-template <typename T> constexpr int VMAX = sizeof(T) == 8 ? 10 : 12;
+constexpr int VMAX = 10;
 
 __host__ __device__ constexpr int rt_pitch(int W) { return W > 1 ? W + 1 : 1; }
 
 template <typename T, bool INV, int R>
 __device__ __forceinline__ void fft_pass(cx<T>* s, int n, int W, int lgW, int Ns, unsigned mg, int nb,
-                                         const cx<T>* __restrict__ tw, cx<T> (&v)[VMAX<T>])
+                                         const cx<T>* __restrict__ tw, cx<T> (&v)[VMAX])
 {
     constexpr int Q = (8 + R - 1) / R;  // butterflies per thread: tiles launch >= n*W/8 threads
-    static_assert(Q * R <= VMAX<T>, "register buffer too small");
+    static_assert(Q * R <= VMAX, "register buffer too small");
     const int items = nb << lgW, pitch = rt_pitch(W);
     const int lstep = nb * pitch, sstep = Ns * pitch;
 #pragma unroll
@@ -337,15 +245,13 @@ __device__ __forceinline__ void fft_pass(cx<T>* s, int n, int W, int lgW, int Ns
     __syncthreads();
 }
 
-// Full transform of the tile (radices 6, 9 and 10 are FP32's: in FP64 their
-// registers cost more occupancy than the saved passes give, 103 to 120
-// registers against 80, y of 576 points 85 -> 116 us a pass).  Caller synchronises before (tile loaded);
+// Full transform of the tile.  Caller synchronises before (tile loaded);
 // the tile is complete and visible to all threads on return.
 template <typename T, bool INV>
 __device__ __forceinline__ void fft_tile(cx<T>* s, const FftSched& sch, int W, int lgW,
                                          const cx<T>* __restrict__ tw)
 {
-    cx<T> v[VMAX<T>];
+    cx<T> v[VMAX];
     int Ns = 1;
     for (int p = 0; p < sch.npass; ++p) {
         const int R = sch.radix[p];
@@ -356,17 +262,7 @@ __device__ __forceinline__ void fft_tile(cx<T>* s, const FftSched& sch, int W, i
             PPF_PASS(3)
             PPF_PASS(4)
             PPF_PASS(5)
-            PPF_PASS(8)
-            default:
-                if constexpr (sizeof(T) == 4) {
-                    switch (R) {
-                        PPF_PASS(6)
-                        PPF_PASS(9)
-                        PPF_PASS(10)
-                        default: break;
-                    }
-                }
-                break;
+            default: fft_pass<T, INV, 8>(s, sch.n, W, lgW, Ns, mg, sch.n / 8, tw, v); break;
 #undef PPF_PASS
         }
         Ns *= R;

@@ -207,7 +207,16 @@ __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn
             auto put = [&](cx<T> V, int kk) {
                 const cx<T> w = ldg(tw_dct + kk);
                 orow[kk] = (T)2 * (w.x * V.x - w.y * V.y);
-                if (kk > 0 && kk < nc) orow[nx - kk] = (T)-2 * (w.x * V.y + w.y * V.x);
+                if (kk > 0 && kk < nc) {
+                    if constexpr (sizeof(T) == 8) {
+                        orow[nx - kk] = (T)-2 * (w.x * V.y + w.y * V.x);
+                    } else {
+                        // FP32 results stay as they are to the bit: the
+                        // conjugate times the table's own twiddle
+                        const cx<T> U = conj(V), w2 = ldg(tw_dct + (nx - kk));
+                        orow[nx - kk] = (T)2 * (w2.x * U.x - w2.y * U.y);
+                    }
+                }
             };
             put(half(a, b, k), k);
             if (kc != k) put(half(b, a, kc), kc);

@@ -13,6 +13,8 @@
 #include "ppf_tma.cuh"
 #include "ppf_y_dev.cuh"
 
+#include <type_traits>
+
 #ifndef PPF_Y_TMA
 #define PPF_Y_TMA 1
 #endif
@@ -41,13 +43,16 @@ struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
 
 // resident CTAs asked of the compile-time y tiles of the DCT and packed-real
 // kinds
-// (run-time tiles: 64 registers at the largest block, so that three 320-thread
-// blocks of a 320-point FP64 tile fit an SM instead of two)
+// (run-time FP64 tiles come in two builds.  WIDE: 64 registers, so that three
+// 320-thread blocks of a 320-point tile fit an SM instead of two: 320 x 320 x
+// 64 211 -> 199 us.  That build spills a few bytes, and a kernel with local
+// memory does not overlap its launch with the previous kernel: 100 x 90 x 33
+// 53 -> 59 us, so grids without several waves of blocks take the other.)
 template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
-template <typename SH> constexpr int y_ctas = SH::CT && SH::NT <= 256 ? 1024 / SH::NT : 2;
+template <typename SH, bool WIDE> constexpr int y_ctas = !SH::CT ? (WIDE ? 2 : 0) : SH::NT <= 256 ? 1024 / SH::NT : 2;
 
-template <typename T, int KIND, typename SH>
-__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+template <typename T, int KIND, typename SH, bool WIDE = false>
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const int* __restrict__ skip)
@@ -57,8 +62,8 @@ __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yfwd(const cx<T>*
                       blockIdx.y);
 }
 
-template <typename T, int KIND, typename SH>
-__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH>) k_yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+template <typename T, int KIND, typename SH, bool WIDE = false>
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
                                                const double* __restrict__ dc_shift, const int* __restrict__ skip)
@@ -346,15 +351,24 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
             err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               skip_flag);
         };
+        // several waves of blocks: more than 1024 threads for each SM
+        const bool wide = !SH::CT && sizeof(T) == 8 && (long)grid.x * grid.y * threads > 1024L * 148;
+        auto pick = [&](auto k) {
+            constexpr int KIND = decltype(k)::value;
+            if constexpr (!SH::CT && sizeof(T) == 8) {
+                if (wide) { go(k_yfwd<T, KIND, SH, true>); return; }
+            }
+            go(k_yfwd<T, KIND, SH>);
+        };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
                 err = launch_y_c2c_pipe<T, false, SH>(in, in_pitch, out, out_pitch,
                                                                                   ncols, g.nz, tw_ny, nullptr,
                                                                                   skip_flag, st, err_bits);
-            else go(k_yfwd<T, Y_C2C, SH>);
+            else pick(std::integral_constant<int, Y_C2C>{});
         }
-        else if (kind == Y_CDCT) go(k_yfwd<T, Y_CDCT, SH>);
-        else go(k_yfwd<T, Y_RPAIR, SH>);
+        else if (kind == Y_CDCT) pick(std::integral_constant<int, Y_CDCT>{});
+        else pick(std::integral_constant<int, Y_RPAIR>{});
     });
     return err;
 }
@@ -378,15 +392,24 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
             err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               dc_shift, skip_flag);
         };
+        // several waves of blocks: more than 1024 threads for each SM
+        const bool wide = !SH::CT && sizeof(T) == 8 && (long)grid.x * grid.y * threads > 1024L * 148;
+        auto pick = [&](auto k) {
+            constexpr int KIND = decltype(k)::value;
+            if constexpr (!SH::CT && sizeof(T) == 8) {
+                if (wide) { go(k_yinv<T, KIND, SH, true>); return; }
+            }
+            go(k_yinv<T, KIND, SH>);
+        };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
                 err = launch_y_c2c_pipe<T, true, SH>(in, in_pitch, out, out_pitch,
                                                                                  ncols, g.nz, tw_ny, dc_shift,
                                                                                  skip_flag, st, err_bits);
-            else go(k_yinv<T, Y_C2C, SH>);
+            else pick(std::integral_constant<int, Y_C2C>{});
         }
-        else if (kind == Y_CDCT) go(k_yinv<T, Y_CDCT, SH>);
-        else go(k_yinv<T, Y_RPAIR, SH>);
+        else if (kind == Y_CDCT) pick(std::integral_constant<int, Y_CDCT>{});
+        else pick(std::integral_constant<int, Y_RPAIR>{});
     });
     return err;
 }

@@ -68,9 +68,21 @@ __device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch
             const cx<T> V = s[tidx<T, SH>(k, l, W)];
             const cx<T> Vp = s[tidx<T, SH>(k == 0 ? 0 : ny - k, l, W)];
             const cx<T> w = ldg(tw_dct + k);
-            const cx<T> p = cmul(w, V), q = cmul(conj(w), Vp);
-            outp[k * op + l] = p + q;
-            if (k > 0 && 2 * k < ny) outp[(ny - k) * op + l] = mk<T>(q.y - p.y, p.x - q.x);
+            if constexpr (sizeof(T) == 8) {
+                const cx<T> p = cmul(w, V), q = cmul(conj(w), Vp);
+                outp[k * op + l] = p + q;
+                if (k > 0 && 2 * k < ny) outp[(ny - k) * op + l] = mk<T>(q.y - p.y, p.x - q.x);
+            } else {
+                // (FP32 results stay as they are to the bit)
+                auto one = [&](cx<T> a, cx<T> b, cx<T> t) {
+                    cx<T> X;
+                    X.x = t.x * (a.x + b.x) - t.y * (a.y - b.y);
+                    X.y = t.x * (a.y + b.y) + t.y * (a.x - b.x);
+                    return X;
+                };
+                outp[k * op + l] = one(V, Vp, w);
+                if (k > 0 && 2 * k < ny) outp[(ny - k) * op + l] = one(Vp, V, ldg(tw_dct + (ny - k)));
+            }
         }
     } else {
         const int my = ny / 2 + 1;
@@ -138,8 +150,20 @@ __device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch
                 if (e == 0) X.x -= shift;
                 const cx<T> Xp = (k == 0) ? mk<T>((T)0, (T)0) : inp[(ny - k) * ip + l];
                 const cx<T> w = ldg(tw_dct + k);
-                Z = cmul(conj(w), mk<T>(X.x + Xp.y, X.y - Xp.x));
-                Zp = cmul(w, mk<T>(X.x - Xp.y, X.y + Xp.x));
+                if constexpr (sizeof(T) == 8) {
+                    Z = cmul(conj(w), mk<T>(X.x + Xp.y, X.y - Xp.x));
+                    Zp = cmul(w, mk<T>(X.x - Xp.y, X.y + Xp.x));
+                } else {
+                    // (FP32 results stay as they are to the bit)
+                    auto one = [&](cx<T> a, cx<T> b, cx<T> t) {
+                        const T c = t.x, sn = -t.y;
+                        const T zax = c * a.x + sn * b.x, zay = sn * a.x - c * b.x;
+                        const T zbx = c * a.y + sn * b.y, zby = sn * a.y - c * b.y;
+                        return mk<T>(zax - zby, zay + zbx);
+                    };
+                    Z = one(X, Xp, w);
+                    if (k > 0) Zp = one(Xp, X, ldg(tw_dct + (ny - k)));
+                }
             }
             s[tidx<T, SH>(k, l, W)] = Z;
             if (k > 0 && 2 * k < ny) s[tidx<T, SH>(ny - k, l, W)] = Zp;
