@@ -278,12 +278,10 @@ int ztab_rows(const ppf_plan* p) { return p->ykind == Y_C2C ? p->my / 2 + 1 : p-
 // 99 us, 256^3 (151) 424 -> 407, 384^3 (491) 1727 -> 1651, 512 x 512 x 128
 // (571) 697 = 697, 512^3 (2282) 2563 -> 2934; others 128 x 128 x 256 (34) 215
 // -> 182, 256^3 real (134) 533 -> 538; cyclic (two tables) 96 x 96 x 200 (29)
-// 244 -> 174, 256 x 256 x 513 (303) 987 -> 1025.  Mixed, one sweep: 256^3 (75)
-// 672 -> 647, 384 x 384 x 192 (123) 1284 -> 1295; real data (an entry is
-// three times its value) 128 x 128 x 256 (17) 377 -> 367, 256^3 (67) 742 -> 764.
-// Mixed solves of tall columns on few cells have no transform long enough to
-// hide the table's chains (128 x 128 x 200 262 -> 274 us, 160^3 348 -> 346,
-// 192^3 529 -> 500), unless the plane is too small to fill the chip (48 x 48
+// 244 -> 174, 256 x 256 x 513 (303) 987 -> 1025.  Mixed, one sweep: 128^3 225 ->
+// 208; real data (an entry is three times its value) 128 x 128 x 256 (17)
+// 377 -> 367.  Mixed solves of tall columns on few cells have no transform long enough to
+// hide the table's chains (128 x 128 x 200 262 -> 274 us), unless the plane is too small to fill the chip (48 x 48
 // x 512 550 -> 297).  The problems of a batch hide their chains behind one
 // another and would pay the tables' bytes: 64 FP64 problems 8.14 -> 8.70 ms.
 long plan_ztab(const ppf_plan* p)

@@ -124,7 +124,7 @@ __device__ __forceinline__ void zcoef(const double* __restrict__ dx3, const doub
 // warps, sm: zprep_smem bytes of shared memory.  The coefficients are formed
 // as in zcoef, the table entries by the reference's Thomas operations in
 // their order (thomas_poisson<Exact>; FP32: k_thomas_fast's).  Bound by the
-// latency of its reciprocal chains (about 0.1 us a row), which the transform
+// latency of its reciprocal chains (about 0.06 us a row), which the transform
 // tiles running beside it hide.
 static __device__ __noinline__ void zprep(const ZPrep& q, unsigned blk, double* sm)
 {

@@ -1124,7 +1124,7 @@ __global__ void __launch_bounds__(32) k_thomas_lowk(void* __restrict__ data_, ZS
 // next chunk load while the current one is swept.  z stage, FP64, with its
 // timing events: 64^3 29 -> 13 us, 128^3 52 -> 19, 256 x 256 x 128 62 -> 47,
 // 384^3 386 -> 286 (k_thomas_exact runs the reciprocal chain twice); cyclic
-// 160 x 128 x 96 66 -> 25; mixed, one sweep, 128^3 67 -> 41, 256^3 165 -> 133.
+// 160 x 128 x 96 66 -> 25; mixed, one sweep, 128^3 67 -> 41.
 constexpr int TAB_TPB = 32;
 constexpr int TAB_C = 16;
 
