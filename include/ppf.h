@@ -151,7 +151,7 @@ PPF_API int ppf_last_sweeps(ppf_plan *plan, int *sweeps, double *last_rel_update
  * synchronises on the recorded events, returns the accumulated
  * milliseconds and launch counts per stage since the last call, and resets
  * them.  Stages (the reference's NVTX ranges, fft_3d_poisson.f90:377-624):
- * 0 z-coefficients, 1 x forward ("Poisson-F_x"), 2 y forward ("-F_y"),
+ * 0 z-coefficients (formed with the first x forward: no time of their own), 1 x forward ("Poisson-F_x"), 2 y forward ("-F_y"),
  * 3 z tridiagonal ("-TDMA-z"), 4 y inverse ("-B_y"), 5 x inverse ("-B_x"),
  * 6 refinement gate, 7 ghost cells. */
 #define PPF_NSTAGES 8

@@ -1,7 +1,7 @@
-"""Run-time transform lengths: every radix of the schedules (FP32 also 6, 9
-and 10), odd half-lengths, the shortest lines and tiles with a ragged last
-line or column, in each pair of boundary conditions, against the oracle with
-the tolerances of the other parity tests."""
+"""Run-time transform lengths: every radix of the schedules, odd half-lengths,
+the shortest lines and tiles with a ragged last line or column, in each pair
+of boundary conditions, against the oracle with the tolerances of the other
+parity tests."""
 import numpy as np
 import pytest
 
