@@ -276,7 +276,7 @@ cudaError_t batch_persistent_grid(size_t smem, int* grid)
     int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = set_smem(k_batch, smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch, BATCH_THREADS, smem);
     if (e != cudaSuccess) return e;
     if (per < 1) return cudaErrorInvalidConfiguration;
@@ -287,7 +287,7 @@ cudaError_t batch_persistent_grid(size_t smem, int* grid)
 cudaError_t launch_batch_persistent(const BProb* probs_d, const BTask* tasks_d, int ntasks, long total_tiles,
                                     int* counters_d, size_t smem, int grid, cudaStream_t st)
 {
-    cudaError_t e = cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = set_smem(k_batch, smem);
     if (e != cudaSuccess) return e;
     k_batch<<<grid, BATCH_THREADS, smem, st>>>(probs_d, tasks_d, ntasks, total_tiles, counters_d);
     return cudaGetLastError();

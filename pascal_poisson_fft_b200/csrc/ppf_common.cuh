@@ -3,6 +3,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 namespace ppf {
 
 template <typename T>
@@ -123,6 +127,47 @@ inline cudaError_t launch_on(void (*kern)(P...), dim3 grid, unsigned threads, si
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
+// Opt a kernel into `bytes` of dynamic shared memory.  The limit belongs to
+// the function, not to a launch, so every host thread shares it: set to each
+// call's size, it could be lowered by a smaller call on another thread between
+// this call's setting and its launch, which is then refused.  It is therefore
+// only ever set to one value and left alone where the 48 KB default (which
+// covers static arrays too) is enough: to the most a block of the kernel can
+// have on the device.
+inline cudaError_t set_smem_most(const void* fn, size_t bytes)
+{
+    struct Size { size_t free, most; };   // without the limit set, and at most
+    static std::map<std::pair<const void*, int>, Size> sizes;
+    static std::mutex mu;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    Size s{ 0, 0 };
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        const auto it = sizes.find({ fn, dev });
+        if (it != sizes.end()) s = it->second;
+    }
+    if (s.most == 0) {
+        int def = 0, optin = 0;
+        cudaFuncAttributes at{};
+        e = cudaDeviceGetAttribute(&def, cudaDevAttrMaxSharedMemoryPerBlock, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
+        if (e != cudaSuccess) return e;
+        s = Size{ (size_t)def - at.sharedSizeBytes, (size_t)optin - at.sharedSizeBytes };
+        std::lock_guard<std::mutex> lk(mu);
+        sizes[{ fn, dev }] = s;
+    }
+    if (bytes <= s.free) return cudaSuccess;
+    if (bytes > s.most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.most);
+}
+template <typename K>
+cudaError_t set_smem(K kern, size_t bytes)
+{
+    return set_smem_most(reinterpret_cast<const void*>(kern), bytes);
+}
 // Per-axis FFT schedule: complex length n = prod(radix[0..npass)).
 struct FftSched {
     int n;

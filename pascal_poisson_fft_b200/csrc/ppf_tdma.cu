@@ -660,7 +660,7 @@ cudaError_t launch_stream(void* data, const ZSys& z, const int* skip, int* err, 
                         (unsigned long long)z.plane * EC * sizeof(float), (unsigned)S::W, (unsigned)S::R))
         return cudaSuccess;
     const size_t smem = S::smem(z.nz, (int)stages);
-    e = cudaFuncSetAttribute(k_thomas_stream<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = set_smem(k_thomas_stream<CPLX>, smem);
     if (e != cudaSuccess) return e;
     // a plane of fewer blocks than SMs leaves most SMs idle behind a few long
     // chains and fences the others off from concurrent work (batched
@@ -1421,10 +1421,8 @@ cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, LSt
     const size_t ks = tab_smem<T, true>(z.nz);
     const bool keep = ks <= 200 * 1024 && (long)nb <= sms * std::min(32L, (long)(227 * 1024 / (ks + 1024)));
     auto go = [&](auto kern, size_t smem) {
-        if (smem > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = set_smem(kern, smem);
+        if (e != cudaSuccess) return e;
         return launch_on(kern, dim3(grid), TAB_TPB, smem, st, data, z, skip, err);
     };
     if constexpr (sizeof(T) == 8)
@@ -1463,9 +1461,8 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
         int dev = 0, sms = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_thomas_lowk<CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_lowk_table, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(3 * sizeof(double) * z.nz));
+        if (e == cudaSuccess) e = set_smem(k_thomas_lowk<CPLX>, lsm);
+        if (e == cudaSuccess) e = set_smem(k_lowk_table, 3 * sizeof(double) * z.nz);
         if (e != cudaSuccess) return e;
         const long groups = (z.plane + 31) / 32;
         const unsigned lg = (unsigned)(groups < sms ? groups : sms);
@@ -1885,7 +1882,7 @@ cudaError_t launch_tdma_sys(const double* a, const double* b, const double* c, d
     const bool many = per >= (cyclic ? 4 : 6) && (cyclic || n_row <= 40);
     if (n_row < 24 || !(few || many)) return cudaSuccess;
     auto go = [&](auto kern) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = set_smem(kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<(unsigned)blocks, 32, smem, st>>>(a, b, c, d, n_sys, n_row);
         return cudaGetLastError();
@@ -1908,16 +1905,12 @@ cudaError_t launch_tdma_many(const double* a, const double* b, const double* c, 
     if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
     dim3 grid((unsigned)(((long)n_sys + TPB - 1) / TPB));
     if (cyclic) {
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(k_thomas_cycl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = set_smem(k_thomas_cycl, smem);
+        if (e != cudaSuccess) return e;
         k_thomas_cycl<<<grid, TPB, smem, st>>>(a, b, c, d, n_sys, n_row);
     } else {
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(k_thomas_arr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        const cudaError_t e = set_smem(k_thomas_arr, smem);
+        if (e != cudaSuccess) return e;
         k_thomas_arr<<<grid, TPB, smem, st>>>(a, b, c, d, n_sys, n_row);
     }
     return cudaGetLastError();

@@ -341,14 +341,14 @@ cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const G
             auto kern = dct ? k_xfwd_prep<T, true, SH> : k_xfwd_prep<T, false, SH>;
             const size_t psmem = std::max(smem, zprep_smem(prep->nz));
             const unsigned nprep = zprep_blocks(*prep, threads);
-            err = set_smem(kern, psmem);
+            err = set_tile_smem<SH>(kern, psmem);
             if (err != cudaSuccess) return;
             err = launch_on(kern, dim3(grid.x + nprep), threads, psmem, st, f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n,
                                                         tw_dct, skip_flag, *prep, nprep);
             return;
         }
         auto go = [&](auto kern) {
-            err = set_smem(kern, smem);
+            err = set_tile_smem<SH>(kern, smem);
             if (err != cudaSuccess) return;
             err = launch_on(kern, grid, threads, smem, st, f, rs, g, out, out_pitch, sch, W, ilog2i(W), tw_half, tw_n, tw_dct,
                                               skip_flag);
@@ -400,7 +400,7 @@ cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, floa
         dim3 grid((unsigned)(((long)g.ny * g.nz + W - 1) / W));
         if (blocks_used) *blocks_used = grid.x;
         auto go = [&](auto kern) {
-            err = set_smem(kern, smem);
+            err = set_tile_smem<SH>(kern, smem);
             if (err != cudaSuccess) return;
             err = launch_on(kern, grid, threads, smem, st, in, in_pitch, P, U, g, partials, mean_prev, sch, W, ilog2i(W), tw_half,
                                               tw_n, tw_dct, skip_flag);
@@ -410,7 +410,7 @@ cudaError_t launch_xinv(bool dct, const void* in, long in_pitch, double* P, floa
                 auto pipe = [&](auto kern, bool bulk) {
                     const size_t rows = bulk ? (size_t)xinv_rs(SH::N) : (size_t)(SH::N + 1);
                     const size_t psmem = 2 * rows * SH::W * sizeof(cx<T>);
-                    err = set_smem(kern, psmem);
+                    err = set_tile_smem<SH>(kern, psmem);
                     unsigned pgrid = 0;
                     if (err == cudaSuccess) err = persistent_grid(kern, SH::NT, psmem, (long)grid.x, &pgrid);
                     if (err != cudaSuccess) return;

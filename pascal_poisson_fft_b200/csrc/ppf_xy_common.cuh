@@ -15,15 +15,19 @@ inline int ilog2i(int w)
     return l;
 }
 
-// Opt a kernel into `bytes` of dynamic shared memory.  The 48 KB default
-// covers static plus dynamic memory, and the transform kernels hold up to
-// 4 KB of static arrays (line tables, reduction slots), so the attribute
-// is set from 40 KB of dynamic memory on.
-template <typename K>
-cudaError_t set_smem(K kern, size_t bytes)
+// set_smem of a transform kernel.  A compile-time tile asks for the same size
+// at every call (its own; the z preparation beside it stays below 40 KB), so
+// its limit is that size; static arrays of the transform kernels take up to
+// 6 KB of the 48 KB default.
+template <typename SH, typename K>
+cudaError_t set_tile_smem(K kern, size_t bytes)
 {
-    if (bytes <= 40 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if constexpr (SH::CT) {
+        if (bytes <= 40 * 1024) return cudaSuccess;
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    } else {
+        return set_smem(kern, bytes);
+    }
 }
 
 // run-time tile shape: W lines (a 128-byte bank row of elements when it

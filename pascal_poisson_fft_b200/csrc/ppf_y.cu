@@ -302,7 +302,7 @@ cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long o
         if (tma) {
             auto kern = k_y_c2c_tma<INV, SH>;
             const size_t smem = 2 * (size_t)SH::N * SH::W * sizeof(cx<T>) + 128;
-            cudaError_t e = set_smem(kern, smem);
+            cudaError_t e = set_tile_smem<SH>(kern, smem);
             if (e != cudaSuccess) return e;
             const long tiles = (long)((ncols + SH::W - 1) / SH::W) * nz;
             unsigned grid = 0;
@@ -323,7 +323,7 @@ cudaError_t launch_y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* out, long o
         else return k_y_c2c_pipe<T, INV, SH, false>;
     }();
     const size_t smem = 2 * (size_t)SH::N * SH::W * sizeof(cx<T>);
-    cudaError_t e = set_smem(kern, smem);
+    cudaError_t e = set_tile_smem<SH>(kern, smem);
     if (e != cudaSuccess) return e;
     const long tiles = (long)((ncols + SH::W - 1) / SH::W) * nz;
     unsigned grid = 0;
@@ -346,7 +346,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         const size_t smem = tile_elems<SH>(g.ny, W) * sizeof(cx<T>);
         dim3 grid((unsigned)((ncols + W - 1) / W), (unsigned)g.nz);
         auto go = [&](auto kern) {
-            err = set_smem(kern, smem);
+            err = set_tile_smem<SH>(kern, smem);
             if (err != cudaSuccess) return;
             err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               skip_flag);
@@ -387,7 +387,7 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         const size_t smem = tile_elems<SH>(g.ny, W) * sizeof(cx<T>);
         dim3 grid((unsigned)((ncols + W - 1) / W), (unsigned)g.nz);
         auto go = [&](auto kern) {
-            err = set_smem(kern, smem);
+            err = set_tile_smem<SH>(kern, smem);
             if (err != cudaSuccess) return;
             err = launch_on(kern, grid, threads, smem, st, in, in_pitch, out, out_pitch, ncols, g, sch, W, ilog2i(W), tw_ny, tw_dct,
                                               dc_shift, skip_flag);
