@@ -93,7 +93,12 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
 // memory, then lets the next kernel's blocks in.  Without the launch
 // attribute both instructions do nothing.  A solve's first launch waits for
 // its predecessor as usual, and its last kernel only waits (pdl_wait): what
-// runs before and after a solve sees ordinary stream order.
+// runs before and after a solve sees ordinary stream order.  What a kernel of
+// the solve wrote (spectra, flags, scalars, partial sums) changes while the
+// next one is already resident, so it is read by ordinary loads through
+// pointers without const __restrict__, which would allow the read-only path
+// and loads moved above the wait; the caller's arrays, twiddles, eigenvalues
+// and the iterate of a sweep (ld_pair_al) keep it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter()
 {

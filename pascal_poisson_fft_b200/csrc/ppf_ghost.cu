@@ -129,7 +129,7 @@ cudaError_t launch_ghosts(double* P, const Geom& g, const double* dmx1, const do
     return launch_on(k_ghosts, dim3((unsigned)std::min(want, 148L * 64)), 256, 0, st, a);
 }
 
-__global__ void __launch_bounds__(512) k_sweep_gate(const double* __restrict__ partials, long nblocks, double ncell,
+__global__ void __launch_bounds__(512) k_sweep_gate(const double* partials, long nblocks, double ncell,
                                                     double* mean_prev, int* skip, int* sweeps_done, double* last_rel,
                                                     double tol, int initial)
 {

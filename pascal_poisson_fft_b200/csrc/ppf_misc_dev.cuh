@@ -60,7 +60,7 @@ __device__ __forceinline__ void ghost_axis(double* __restrict__ P, int dir, int 
 // gate for the remaining sweeps once it is below tol.  A sweep that was
 // skipped (gate already closed) leaves everything unchanged.
 // (one CTA of a power-of-two size up to 512 threads)
-__device__ __forceinline__ void sweep_gate(const double* __restrict__ partials, long nblocks, double ncell,
+__device__ __forceinline__ void sweep_gate(const double* partials, long nblocks, double ncell,
                                            double* mean_prev, int* skip, int* sweeps_done, double* last_rel,
                                            double tol, int initial)
 {

@@ -82,7 +82,7 @@ bool tma_map_2d_f32(CUtensorMap* map, void* base, unsigned long long inner, unsi
 // MODE 0: every system, arithmetic A.  MODE 1: only systems above the
 // low-wavenumber threshold (FP32 path).  MODE 2: only systems below it.
 template <typename T, typename A, bool CPLX, int MODE, bool CYC>
-__global__ void __launch_bounds__(TPB) k_thomas_z(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
+__global__ void __launch_bounds__(TPB) k_thomas_z(void* data_, ZSys z, const int* skip,
                                                   int* __restrict__ err)
 {
     pdl_enter();
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(TPB) k_thomas_z(void* __restrict__ data_, ZSys
     co.ly = z.lamy[ky];
     co.pin = (kx == 0 && ky == 0);
     if (MODE != 0) {
-        const bool low = (co.lx + co.ly) * __ldg(z.dzmin2) < z.lowk;
+        const bool low = (co.lx + co.ly) * *z.dzmin2 < z.lowk;
         if ((MODE == 1) == low) return;
     }
     double zsum = 0.0;
@@ -680,7 +680,7 @@ cudaError_t launch_stream(void* data, const ZSys& z, const int* skip, int* err, 
 // level) and, with PREF, the next chunk's rows loaded while the current one
 // is eliminated.
 template <bool CPLX, bool PREF>
-__global__ void __launch_bounds__(TPB) k_thomas_exact(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
+__global__ void __launch_bounds__(TPB) k_thomas_exact(void* data_, ZSys z, const int* skip,
                                                       int* __restrict__ err)
 {
     pdl_enter();
@@ -1276,7 +1276,7 @@ size_t tab_smem(int nz)
 }
 
 template <typename T, bool CPLX, bool KEEP>
-__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* __restrict__ data_, ZSys z, const int* __restrict__ skip,
+__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* data_, ZSys z, const int* skip,
                                                         int* __restrict__ err)
 {
     pdl_enter();
@@ -1297,7 +1297,7 @@ __global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* __restrict__ data_
     const int kx = (int)(sys % (unsigned)z.pitch), ky = (int)(sys / (unsigned)z.pitch);
     const bool in = kx < z.mx && ky < z.my;
     const double lx = in ? z.lamx[kx] : 0.0, ly = in ? z.lamy[ky] : 0.0;
-    const bool high = sizeof(T) == 4 && in && !((lx + ly) * __ldg(z.dzmin2) < z.lowk);
+    const bool high = sizeof(T) == 4 && in && !((lx + ly) * *z.dzmin2 < z.lowk);
     const bool mine = in && high == fp32;
     if (!__any_sync(0xffffffffu, mine)) return;
     for (int k = threadIdx.x; k < nz; k += TAB_TPB) {
@@ -1341,8 +1341,8 @@ __global__ void __launch_bounds__(TAB_TPB) k_thomas_tab(void* __restrict__ data_
 // 1 .. nz-1 are solved for y in place, x_0 follows from their ends and the
 // tabulated e, then x_k = y_k + x_0 e_k.
 template <bool CPLX, bool KEEP>
-__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab_cyc(void* __restrict__ data_, ZSys z,
-                                                            const int* __restrict__ skip, int* __restrict__ err)
+__global__ void __launch_bounds__(TAB_TPB) k_thomas_tab_cyc(void* data_, ZSys z,
+                                                            const int* skip, int* __restrict__ err)
 {
     pdl_enter();
     if (skip && *skip) return;

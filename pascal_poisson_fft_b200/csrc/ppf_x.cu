@@ -27,7 +27,7 @@ namespace ppf {
 #define PPF_XFWD_PARAMS                                                                                      \
     const double* __restrict__ f, ResidIn rs, Geom g, void* __restrict__ out_, long out_pitch, FftSched sch,    \
         int Wrt, int lgWrt, const cx<T>* __restrict__ tw_half, const cx<T>* __restrict__ tw_n,                \
-        const cx<T>* __restrict__ tw_dct, const int* __restrict__ skip
+        const cx<T>* __restrict__ tw_dct, const int* skip
 #define PPF_XFWD_ARGS(tile) f, rs, g, out_, out_pitch, sch, Wrt, lgWrt, tw_half, tw_n, tw_dct, skip, tile
 
 // FP64 compile-time tiles: resident CTAs per SM asked of the compiler.  Five
@@ -72,11 +72,11 @@ __global__ void __launch_bounds__(SH::NT, x64_ctas(SH::NT)) k_xfwd64(PPF_XFWD_PA
 // tile's interior values are written and visible to the block: the value a
 // ghost receives is the one just stored, in every iterate kind.
 #define PPF_XINV_PARAMS                                                                                      \
-    const void* __restrict__ in_, long in_pitch, double* __restrict__ P, float* __restrict__ U, Geom g,        \
+    const void* in_, long in_pitch, double* __restrict__ P, float* U, Geom g,        \
         double* __restrict__ partials,                                                                         \
-        const double* __restrict__ mean_prev, FftSched sch, int Wrt, int lgWrt,                                \
+        const double* mean_prev, FftSched sch, int Wrt, int lgWrt,                                \
         const cx<T>* __restrict__ tw_half, const cx<T>* __restrict__ tw_n, const cx<T>* __restrict__ tw_dct,   \
-        const int* __restrict__ skip
+        const int* skip
 #define PPF_XINV_ARGS in_, in_pitch, P, U, g, partials, mean_prev, sch, Wrt, lgWrt, tw_half, tw_n, tw_dct, skip, \
     (long)blockIdx.x
 
@@ -116,12 +116,12 @@ constexpr unsigned XB_POLL_NS = 20000;
 constexpr long XB_WAIT_LIMIT = 100000;
 
 template <typename T, bool ACC, bool GHOST, typename SH, int UK = U_P, bool BULK = false>
-__global__ void __launch_bounds__(SH::NT, (SH::N <= 128) ? 2 : SH::N == 384 ? 3 : (SH::N == 256 ? PPF_XINV_256_CTAS : 0)) k_xinv_pipe(const cx<T>* __restrict__ in, long in_pitch,
-                                                     double* __restrict__ P, float* __restrict__ U, Geom g,
+__global__ void __launch_bounds__(SH::NT, (SH::N <= 128) ? 2 : SH::N == 384 ? 3 : (SH::N == 256 ? PPF_XINV_256_CTAS : 0)) k_xinv_pipe(const cx<T>* in, long in_pitch,
+                                                     double* __restrict__ P, float* U, Geom g,
                                                      double* __restrict__ partials,
-                                                     const double* __restrict__ mean_prev,
+                                                     const double* mean_prev,
                                                      const cx<T>* __restrict__ tw_half,
-                                                     const cx<T>* __restrict__ tw_n, const int* __restrict__ skip,
+                                                     const cx<T>* __restrict__ tw_n, const int* skip,
                                                      int* __restrict__ err)
 {
     pdl_enter();

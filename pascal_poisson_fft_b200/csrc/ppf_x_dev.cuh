@@ -47,8 +47,11 @@ __device__ __forceinline__ void prefetch_row(const U* base, long o, int n)
 }
 
 // the two values at p, p+1 (p 16-byte aligned for FP64, 8-byte for FP32);
-// NC: through the read-only cache (only for data no earlier part of the
-// same kernel launch wrote)
+// NC: through the read-only path, for data that neither this launch nor the
+// previous kernel of the solve writes.  That holds for the iterate of a
+// refinement sweep: the gate stands between the x inverse that wrote it and
+// the x forward, and lets the x forward's blocks in only after its own wait
+// for the x inverse (ordinary loads: x forward of 512 x 512 x 256 +2 %)
 template <bool NC>
 __device__ __forceinline__ void ld_pair_al(const double* p, double& a, double& b)
 {
@@ -74,7 +77,7 @@ template <typename T, bool DCT, int RESID, typename SH, bool NC = true>
 __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn& rs, const Geom& g,
                                      void* __restrict__ out_, long out_pitch, const FftSched& sch, int Wrt, int lgWrt,
                                      const cx<T>* __restrict__ tw_half, const cx<T>* __restrict__ tw_n,
-                                     const cx<T>* __restrict__ tw_dct, const int* __restrict__ skip, long tile)
+                                     const cx<T>* __restrict__ tw_dct, const int* skip, long tile)
 {
     if (skip && *skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -225,7 +228,7 @@ __device__ __forceinline__ void xfwd(const double* __restrict__ f, const ResidIn
 }
 
 template <int UK>
-__device__ __forceinline__ void x_ghosts(double* __restrict__ P, float* __restrict__ U, const Geom& g, long line0,
+__device__ __forceinline__ void x_ghosts(double* __restrict__ P, float* U, const Geom& g, long line0,
                                          int W, long nlines, int nx)
 {
     for (int t = threadIdx.x; t < 2 * W; t += blockDim.x) {
@@ -247,11 +250,11 @@ __device__ __forceinline__ void x_ghosts(double* __restrict__ P, float* __restri
 // (values that are FP32 numbers already), U_ACC reads u from U and writes P.
 // --------------------------------------------------------------------------
 template <typename T, bool DCT, bool ACC, bool GHOST, typename SH, int UK = U_P>
-__device__ __forceinline__ void xinv(const void* __restrict__ in_, long in_pitch, double* __restrict__ P,
-                                     float* __restrict__ U, const Geom& g, double* __restrict__ partials,
-                                     const double* __restrict__ mean_prev, const FftSched& sch, int Wrt, int lgWrt,
+__device__ __forceinline__ void xinv(const void* in_, long in_pitch, double* __restrict__ P,
+                                     float* U, const Geom& g, double* __restrict__ partials,
+                                     const double* mean_prev, const FftSched& sch, int Wrt, int lgWrt,
                                      const cx<T>* __restrict__ tw_half, const cx<T>* __restrict__ tw_n,
-                                     const cx<T>* __restrict__ tw_dct, const int* __restrict__ skip, long tile)
+                                     const cx<T>* __restrict__ tw_dct, const int* skip, long tile)
 {
     if (skip && *skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];

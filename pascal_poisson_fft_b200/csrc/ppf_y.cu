@@ -52,10 +52,10 @@ template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
 template <typename SH, bool WIDE> constexpr int y_ctas = !SH::CT ? (WIDE ? 2 : 0) : SH::NT <= 256 ? 1024 / SH::NT : 2;
 
 template <typename T, int KIND, typename SH, bool WIDE = false>
-__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yfwd(const cx<T>* in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
-                                               const int* __restrict__ skip)
+                                               const int* skip)
 {
     pdl_enter();
     yfwd<T, KIND, SH>(in, in_pitch, out, out_pitch, ncols, g, sch, Wrt, lgWrt, tw_ny, tw_dct, skip, blockIdx.x,
@@ -63,10 +63,10 @@ __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yfwd(const 
 }
 
 template <typename T, int KIND, typename SH, bool WIDE = false>
-__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yinv(const cx<T>* in, long in_pitch, cx<T>* __restrict__ out,
                                                long out_pitch, int ncols, Geom g, FftSched sch, int Wrt, int lgWrt,
                                                const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
-                                               const double* __restrict__ dc_shift, const int* __restrict__ skip)
+                                               const double* dc_shift, const int* skip)
 {
     pdl_enter();
     yinv<T, KIND, SH>(in, in_pitch, out, out_pitch, ncols, g, sch, Wrt, lgWrt, tw_ny, tw_dct, dc_shift, skip,
@@ -84,9 +84,9 @@ __global__ void __launch_bounds__(y_threads<SH>, y_ctas<SH, WIDE>) k_yinv(const 
 // unswizzled, copied in 16-byte pairs of columns, and transformed by the
 // paired passes (fft_pass_pair), which also store column pairs.
 template <typename T, bool INV, typename SH, bool PAIR>
-__device__ __forceinline__ void y_c2c_pipe(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__device__ __forceinline__ void y_c2c_pipe(const cx<T>* in, long in_pitch, cx<T>* __restrict__ out,
                                            long out_pitch, int ncols, int nz, const cx<T>* __restrict__ tw,
-                                           const double* __restrict__ dc_shift, const int* __restrict__ skip)
+                                           const double* dc_shift, const int* skip)
 {
     if (skip && *skip) return;
     constexpr int N = SH::N, W = SH::W, NT = SH::NT;
@@ -184,8 +184,8 @@ template <bool INV, typename SH>
 __global__ void __launch_bounds__(SH::NT, 1) k_y_c2c_tma(const __grid_constant__ CUtensorMap tmap,
                                                      cx<float>* __restrict__ out, long out_pitch, int ncols, int nz,
                                                      const cx<float>* __restrict__ tw,
-                                                     const double* __restrict__ dc_shift,
-                                                     const int* __restrict__ skip, int* __restrict__ err)
+                                                     const double* dc_shift,
+                                                     const int* skip, int* __restrict__ err)
 {
     pdl_enter();
     if (skip && *skip) return;
@@ -261,11 +261,11 @@ __global__ void __launch_bounds__(SH::NT, 1) k_y_c2c_tma(const __grid_constant__
 
 // FP32 tiles: one CTA per SM (two 64 KB buffers at 512 threads)
 template <typename T, bool INV, typename SH, bool PAIR>
-__global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* __restrict__ in, long in_pitch,
+__global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* in, long in_pitch,
                                                       cx<T>* __restrict__ out, long out_pitch, int ncols, int nz,
                                                       const cx<T>* __restrict__ tw,
-                                                      const double* __restrict__ dc_shift,
-                                                      const int* __restrict__ skip)
+                                                      const double* dc_shift,
+                                                      const int* skip)
 {
     pdl_enter();
     y_c2c_pipe<T, INV, SH, PAIR>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip);
@@ -275,11 +275,11 @@ __global__ void __launch_bounds__(SH::NT) k_y_c2c_pipe(const cx<T>* __restrict__
 // bounds the registers to 85 a thread; two of the 384-thread shapes (three
 // left 56 registers and 200 bytes of spills)
 template <bool INV, typename SH>
-__global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 768 / SH::NT) k_y_c2c_pipe64(const cx<double>* __restrict__ in, long in_pitch,
+__global__ void __launch_bounds__(SH::NT, SH::NT > 256 ? 2 : 768 / SH::NT) k_y_c2c_pipe64(const cx<double>* in, long in_pitch,
                                                            cx<double>* __restrict__ out, long out_pitch, int ncols,
                                                            int nz, const cx<double>* __restrict__ tw,
-                                                           const double* __restrict__ dc_shift,
-                                                           const int* __restrict__ skip)
+                                                           const double* dc_shift,
+                                                           const int* skip)
 {
     pdl_enter();
     y_c2c_pipe<double, INV, SH, false>(in, in_pitch, out, out_pitch, ncols, nz, tw, dc_shift, skip);

@@ -18,10 +18,10 @@ namespace ppf {
 constexpr int ct_log2y(int w) { return w <= 1 ? 0 : 1 + ct_log2y(w / 2); }
 
 template <typename T, int KIND, typename SH>
-__device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__device__ __forceinline__ void yfwd(const cx<T>* in, long in_pitch, cx<T>* __restrict__ out,
                                      long out_pitch, int ncols, const Geom& g, const FftSched& sch, int Wrt, int lgWrt,
                                      const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
-                                     const int* __restrict__ skip, int cblk, int z)
+                                     const int* skip, int cblk, int z)
 {
     if (skip && *skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -103,10 +103,10 @@ __device__ __forceinline__ void yfwd(const cx<T>* __restrict__ in, long in_pitch
 }
 
 template <typename T, int KIND, typename SH>
-__device__ __forceinline__ void yinv(const cx<T>* __restrict__ in, long in_pitch, cx<T>* __restrict__ out,
+__device__ __forceinline__ void yinv(const cx<T>* in, long in_pitch, cx<T>* __restrict__ out,
                                      long out_pitch, int ncols, const Geom& g, const FftSched& sch, int Wrt, int lgWrt,
                                      const cx<T>* __restrict__ tw_ny, const cx<T>* __restrict__ tw_dct,
-                                     const double* __restrict__ dc_shift, const int* __restrict__ skip, int cblk,
+                                     const double* dc_shift, const int* skip, int cblk,
                                      int z)
 {
     if (skip && *skip) return;
