@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 # system beside them; run-time lengths; FP64 with checkpoints
 CASES = [((48, 40, 33), (1, 1, 1), PPF_MIXED), ((256, 160, 64), (1, 1, 0), PPF_MIXED),
          ((128, 128, 200), (1, 1, 0), PPF_MIXED), ((300, 180, 48), (0, 0, 0), PPF_FP32),
-         ((256, 250, 180), (0, 0, 0), PPF_FP64)]
+         ((256, 250, 200), (0, 0, 0), PPF_FP64)]
 
 
 @pytest.mark.parametrize("case", CASES)
