@@ -147,13 +147,15 @@ PPF_API int ppf_solve_host_async(ppf_plan *plan, const double *f_h, double *p_h,
 PPF_API int ppf_last_sweeps(ppf_plan *plan, int *sweeps, double *last_rel_update, void *stream);
 
 /* Per-stage device timing.  While enabled, every solve records a CUDA
- * event after each kernel on the solve's stream; ppf_stage_times()
+ * event after each stage's launches on the solve's stream; ppf_stage_times()
  * synchronises on the recorded events, returns the accumulated
- * milliseconds and launch counts per stage since the last call, and resets
+ * milliseconds and kernel launches per stage since the last call, and resets
  * them.  Stages (the reference's NVTX ranges, fft_3d_poisson.f90:377-624):
- * 0 z-coefficients (formed with the first x forward: no time of their own), 1 x forward ("Poisson-F_x"), 2 y forward ("-F_y"),
- * 3 z tridiagonal ("-TDMA-z"), 4 y inverse ("-B_y"), 5 x inverse ("-B_x"),
- * 6 refinement gate, 7 ghost cells. */
+ * 0 z-coefficients and the list of low wavenumbers (a plan with z tables forms
+ * them in the first x forward: no launch and no time of their own),
+ * 1 x forward ("Poisson-F_x"), 2 y forward ("-F_y"), 3 z tridiagonal
+ * ("-TDMA-z"), 4 y inverse ("-B_y"), 5 x inverse ("-B_x"), 6 refinement gate,
+ * 7 ghost cells. */
 #define PPF_NSTAGES 8
 PPF_API int ppf_stage_timing(ppf_plan *plan, int enable);
 PPF_API int ppf_stage_times(ppf_plan *plan, double *ms, int *launches);

@@ -181,7 +181,8 @@ struct ppf_plan {
     double* slab_part = nullptr;   // interior partial sums of ppf_slab_sum (allocated on first use)
     // per-stage timing (ppf_stage_timing)
     bool timing = false;
-    std::vector<std::pair<int, cudaEvent_t>> marks;   // stage id (-1 = start), event
+    struct Mark { int stage, launches; cudaEvent_t ev; };   // stage -1: start
+    std::vector<Mark> marks;
 };
 
 namespace {
@@ -212,18 +213,18 @@ int upload_twiddles(ppf_plan* p)
 
 void drop_marks(ppf_plan* p)
 {
-    for (auto& m : p->marks) cudaEventDestroy(m.second);
+    for (auto& m : p->marks) cudaEventDestroy(m.ev);
     p->marks.clear();
 }
 
-// records an event after a stage's launch when timing is enabled
-void mark(ppf_plan* p, int stage, cudaStream_t st)
+// records an event after a stage's launches when timing is enabled
+void mark(ppf_plan* p, int stage, cudaStream_t st, int launches = 1)
 {
     if (!p->timing) return;
     cudaEvent_t ev;
     if (cudaEventCreate(&ev) != cudaSuccess) return;
     cudaEventRecord(ev, st);
-    p->marks.emplace_back(stage, ev);
+    p->marks.push_back({ stage, launches, ev });
 }
 
 void free_plan(ppf_plan* p)
@@ -483,16 +484,25 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
         zp.tab = p->ztab; zp.tplane = z.tplane; zp.lowk = z.lowk;
         zp.f32 = sizeof(T) == 4; zp.cyclic = p->g.pz;
     }
-    cudaError_t e = launch_xfwd<T>(p->xdct, f, resid ? &rs : nullptr, p->g, p->A, p->a_pitch, p->sx, txh, txn, txd,
-                                   skip, resid ? st : LStream(st.s), resid ? nullptr : &zp);
+    cudaError_t e;
+    if (!resid && !z.tab) {
+        // without tables to fill beside the transform, in a launch of its own
+        e = launch_zprep(zp, LStream(st.s));
+        if (e != cudaSuccess) return cuda_fail(e, "z coefficients");
+        mark(p, 0, st);
+    }
+    e = launch_xfwd<T>(p->xdct, f, resid ? &rs : nullptr, p->g, p->A, p->a_pitch, p->sx, txh, txn, txd, skip,
+                       resid ? st : LStream(st.s), !resid && z.tab ? &zp : nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "x forward");
+    mark(p, 1, st);
     if (!resid && z.lowk_list) {
         // the FP64 low-|k| set of this solve (flags[3], zeroed with the
         // flags, counts it); the z solve of every pass uses it
-        e = launch_lowk_list(z, st);
+        int n = 0;
+        e = launch_lowk_list(z, st, &n);
         if (e != cudaSuccess) return cuda_fail(e, "low-|k| list");
+        if (n) mark(p, 0, st, n);
     }
-    mark(p, 1, st);
     // complex views of A and B for the y pass
     const long a_cp = p->xdct ? p->a_pitch / 2 : p->a_pitch;
     const long b_cp = (p->xdct && p->ydct) ? p->b_pitch / 2 : p->b_pitch;
@@ -503,11 +513,12 @@ int run_pass(ppf_plan* p, const double* f, double* P, bool resid, bool accumulat
     mark(p, 2, st);
     // the z solve of FP32 spectra without tables forks to the auxiliary stream
     const bool fork = sizeof(T) == 4 && !z.tab;
-    const ZStreams zs{ fork ? LStream(st.s) : st, p->aux, p->ev_fork, p->ev_join };
+    int zn = 1;
+    const ZStreams zs{ fork ? LStream(st.s) : st, p->aux, p->ev_fork, p->ev_join, &zn };
     e = p->cplx ? launch_tdma_z<T, true>(p->B, z, skip, p->flags + 2, zs)
                 : launch_tdma_z<T, false>(p->B, z, skip, p->flags + 2, zs);
     if (e != cudaSuccess) return cuda_fail(e, "z tridiagonal");
-    mark(p, 3, st);
+    mark(p, 3, st, zn);
     e = launch_yinv<T>(p->ykind, reinterpret_cast<const cx<T>*>(p->B), b_cp, reinterpret_cast<cx<T>*>(p->A), a_cp,
                        p->ycols, p->g, p->sy, tyn, tyd, p->scal + 4, skip, fork ? LStream(st.s) : st, p->flags + 2);
     if (e != cudaSuccess) return cuda_fail(e, "y inverse");
@@ -717,15 +728,15 @@ int ppf_stage_times(ppf_plan* plan, double* ms, int* launches)
     for (int i = 0; i < PPF_NSTAGES; ++i) { ms[i] = 0.0; launches[i] = 0; }
     cudaEvent_t prev = nullptr;
     for (auto& m : plan->marks) {
-        cudaError_t e = cudaEventSynchronize(m.second);
+        cudaError_t e = cudaEventSynchronize(m.ev);
         if (e != cudaSuccess) { drop_marks(plan); return cuda_fail(e, "event synchronise"); }
-        if (m.first >= 0 && prev) {
+        if (m.stage >= 0 && prev) {
             float t = 0.f;
-            cudaEventElapsedTime(&t, prev, m.second);
-            ms[m.first] += t;
-            launches[m.first] += 1;
+            cudaEventElapsedTime(&t, prev, m.ev);
+            ms[m.stage] += t;
+            launches[m.stage] += m.launches;
         }
-        prev = m.second;
+        prev = m.ev;
     }
     drop_marks(plan);
     return PPF_OK;

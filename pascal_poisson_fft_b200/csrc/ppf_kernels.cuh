@@ -151,6 +151,7 @@ struct ZStreams {
     LStream st;
     cudaStream_t aux;
     cudaEvent_t fork, join;
+    int* launches = nullptr;   // set to the number of kernels launched
 };
 
 template <typename T, bool CPLX>
@@ -158,7 +159,8 @@ cudaError_t launch_tdma_z(void* data, const ZSys& z, const int* skip_flag, int* 
 
 // the low-|k| system list of a mixed or FP32 solve (z.lowk_list), once per
 // solve before its first z solve; a no-op where the list is not used
-cudaError_t launch_lowk_list(const ZSys& z, LStream st);
+// (launches: the number of kernels launched)
+cudaError_t launch_lowk_list(const ZSys& z, LStream st, int* launches = nullptr);
 
 // ---- ghost cells (ppf_ghost.cu) ----
 // zfaces: z faces to fill (1 lower, 2 upper; 3 for a whole domain, the

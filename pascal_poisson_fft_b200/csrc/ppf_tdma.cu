@@ -1454,6 +1454,7 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
         if (e != cudaSuccess) return e;
         lo = zs.aux;
     }
+    int launches = 2;   // the low-|k| systems and the bulk
     const size_t lsm = lowk_smem<CPLX>(z.nz);
     if (!CYC && lowk_listed(z) && lsm <= 160 * 1024) {
         // persistent one-warp blocks (one per SM) over the list; the first
@@ -1466,8 +1467,10 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
         if (e != cudaSuccess) return e;
         const long groups = (z.plane + 31) / 32;
         const unsigned lg = (unsigned)(groups < sms ? groups : sms);
-        if (z.lowk_tab && z.lowk_build)
+        if (z.lowk_tab && z.lowk_build) {
             k_lowk_table<<<lg, 32, 3 * sizeof(double) * z.nz, lo>>>(z, skip);
+            ++launches;
+        }
         k_thomas_lowk<CPLX><<<lg, 32, lsm, lo>>>(data, z, skip, err);
     } else {
         k_thomas_z<float, Exact, CPLX, 2, CYC><<<grid, TPB, 0, lo>>>(data, z, skip, err);
@@ -1488,13 +1491,15 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
         if (e == cudaSuccess) e = cudaStreamWaitEvent(zs.st.s, zs.join, 0);
         if (e != cudaSuccess) return e;
     }
+    if (zs.launches) *zs.launches = launches;
     return cudaGetLastError();
 }
 }  // namespace
 
-cudaError_t launch_lowk_list(const ZSys& z, LStream st)
+cudaError_t launch_lowk_list(const ZSys& z, LStream st, int* launches)
 {
     if (!lowk_listed(z)) return cudaSuccess;
+    if (launches) *launches = 1;
     k_lowk_list<<<(unsigned)((z.plane + 255) / 256), 256, 0, st.s>>>(z);
     return cudaGetLastError();
 }

@@ -324,11 +324,6 @@ cudaError_t launch_xfwd(bool dct, const double* f, const ResidIn* resid, const G
     ResidIn rs{};
     if (resid) rs = *resid;
     if (resid && prep) return cudaErrorInvalidValue;
-    if (prep && !prep->tab) {
-        const cudaError_t e = launch_zprep(*prep, st);
-        if (e != cudaSuccess) return e;
-        prep = nullptr;
-    }
     cudaError_t err = cudaSuccess;
     with_shape<T>(sch, [&](auto sh) {
         using SH = decltype(sh);
