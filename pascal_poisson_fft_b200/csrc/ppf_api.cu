@@ -297,7 +297,9 @@ long plan_ztab(const ppf_plan* p)
     const long cells = (long)p->g.nx * p->g.ny * p->g.nz;
     // where the streamed FP32 bulk would run its twisted sweep (a block of 256
     // values for every SM), whose roundings the tables' sweep does not share
-    if (f32 && p->b_pitch * (long)p->my * (p->cplx ? 2 : 1) >= 147L * 256) return 0;
+    int sms = 0;
+    if (f32 && (device_sms(&sms) != cudaSuccess || p->b_pitch * (long)p->my * (p->cplx ? 2 : 1) >= (sms - 1) * 256L))
+        return 0;
     if (f32 && p->g.nz > 160 && cells < 5000000 && p->b_pitch * (long)p->my > 4096) return 0;
     if (field > (mb << 20)) return 0;
     return ztab_doubles(p->g.nz, p->b_pitch * (long)ztab_rows(p), p->g.pz, f32);

@@ -132,6 +132,14 @@ inline cudaError_t launch_on(void (*kern)(P...), dim3 grid, unsigned threads, si
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
+// SMs of the current device
+inline cudaError_t device_sms(int* sms)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
+}
+
 // Opt a kernel into `bytes` of dynamic shared memory.  The limit belongs to
 // the function, not to a launch, so every host thread shares it: set to each
 // call's size, it could be lowered by a smaller call on another thread between

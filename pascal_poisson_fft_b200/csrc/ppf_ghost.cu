@@ -126,7 +126,10 @@ cudaError_t launch_ghosts(double* P, const Geom& g, const double* dmx1, const do
     a.count[1] = 2L * g.nx * (g.nz + 2);
     a.count[2] = (long)((zfaces & 1) + (zfaces >> 1)) * g.nx * g.ny;
     const long want = (a.count[0] + a.count[1] + a.count[2] + 255) / 256;
-    return launch_on(k_ghosts, dim3((unsigned)std::min(want, 148L * 64)), 256, 0, st, a);
+    int sms = 0;
+    const cudaError_t e = device_sms(&sms);
+    if (e != cudaSuccess) return e;
+    return launch_on(k_ghosts, dim3((unsigned)std::min(want, 64L * sms)), 256, 0, st, a);
 }
 
 __global__ void __launch_bounds__(512) k_sweep_gate(const double* partials, long nblocks, double ncell,

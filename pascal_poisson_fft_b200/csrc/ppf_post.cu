@@ -66,7 +66,10 @@ cudaError_t launch_cell_to_node(const double* P, int n1m, int n2m, int n3m, cons
 {
     const long total = (long)n1m * n2m * n3m;
     const long want = (total + 255) / 256;
-    const int blocks = (int)(want < 148L * 32 ? want : 148L * 32);
+    int sms = 0;
+    const cudaError_t e = device_sms(&sms);
+    if (e != cudaSuccess) return e;
+    const int blocks = (int)(want < 32L * sms ? want : 32L * sms);
     k_cell_to_node<<<blocks, 256, 0, st>>>(P, n1m, n2m, n3m, dx1, dx2, dx3, G);
     return cudaGetLastError();
 }

@@ -133,7 +133,10 @@ cudaError_t launch_slab_sum(const double* P, const Geom& g, double* part, double
 cudaError_t launch_slab_shift(double* P, const Geom& g, const double* shift, cudaStream_t st)
 {
     const long total = (long)g.nx * g.ny * g.nz;
-    const unsigned blocks = (unsigned)std::min<long>((total + SL_TPB - 1) / SL_TPB, 148L * 16);
+    int sms = 0;
+    const cudaError_t e = device_sms(&sms);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)std::min<long>((total + SL_TPB - 1) / SL_TPB, 16L * sms);
     k_slab_shift<<<blocks, SL_TPB, 0, st>>>(P, g.nx, g.ny, g.nz, g.pstride_y, g.pstride_z, shift);
     return cudaGetLastError();
 }

@@ -1414,9 +1414,8 @@ cudaError_t launch_tab(const ZSys& z, void* data, const int* skip, int* err, LSt
     // d' in shared memory where every block is resident at once with it (the
     // 227 KB of each SM's shared memory, 1 KB a block reserved): 48 x 48 x 512
     // z 52 -> 43 us; more blocks than that would run in waves
-    int dev = 0, sms = 0;
-    cudaError_t de = cudaGetDevice(&dev);
-    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    const cudaError_t de = device_sms(&sms);
     if (de != cudaSuccess) return de;
     const size_t ks = tab_smem<T, true>(z.nz);
     const bool keep = ks <= 200 * 1024 && (long)nb <= sms * std::min(32L, (long)(227 * 1024 / (ks + 1024)));
@@ -1459,9 +1458,8 @@ cudaError_t launch_z(float*, const ZSys& z, void* data, const int* skip, int* er
     if (!CYC && lowk_listed(z) && lsm <= 160 * 1024) {
         // persistent one-warp blocks (one per SM) over the list; the first
         // pass of a solve fills the coefficient table before
-        int dev = 0, sms = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        int sms = 0;
+        cudaError_t e = device_sms(&sms);
         if (e == cudaSuccess) e = set_smem(k_thomas_lowk<CPLX>, lsm);
         if (e == cudaSuccess) e = set_smem(k_lowk_table, 3 * sizeof(double) * z.nz);
         if (e != cudaSuccess) return e;
@@ -1873,9 +1871,8 @@ cudaError_t launch_tdma_sys(const double* a, const double* b, const double* c, d
                             bool cyclic, cudaStream_t st, bool* used)
 {
     *used = false;
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    cudaError_t e = device_sms(&sms);
     if (e != cudaSuccess) return e;
     const long blocks = ((long)n_sys + 31) / 32;
     const size_t one = (size_t)n_row * 32 * sizeof(double);

@@ -352,7 +352,13 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
                                               skip_flag);
         };
         // several waves of blocks: more than 1024 threads for each SM
-        const bool wide = !SH::CT && sizeof(T) == 8 && (long)grid.x * grid.y * threads > 1024L * 148;
+        bool wide = false;
+        if constexpr (!SH::CT && sizeof(T) == 8) {
+            int sms = 0;
+            err = device_sms(&sms);
+            if (err != cudaSuccess) return;
+            wide = (long)grid.x * grid.y * threads > 1024L * sms;
+        }
         auto pick = [&](auto k) {
             constexpr int KIND = decltype(k)::value;
             if constexpr (!SH::CT && sizeof(T) == 8) {
@@ -393,7 +399,13 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
                                               dc_shift, skip_flag);
         };
         // several waves of blocks: more than 1024 threads for each SM
-        const bool wide = !SH::CT && sizeof(T) == 8 && (long)grid.x * grid.y * threads > 1024L * 148;
+        bool wide = false;
+        if constexpr (!SH::CT && sizeof(T) == 8) {
+            int sms = 0;
+            err = device_sms(&sms);
+            if (err != cudaSuccess) return;
+            wide = (long)grid.x * grid.y * threads > 1024L * sms;
+        }
         auto pick = [&](auto k) {
             constexpr int KIND = decltype(k)::value;
             if constexpr (!SH::CT && sizeof(T) == 8) {
