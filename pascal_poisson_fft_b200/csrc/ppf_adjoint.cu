@@ -155,28 +155,33 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_rhs(const double* g, double* h,
 }
 
 // df = dx3_k * W + c_k (W: ghosted solution of the scaled right-hand side);
-// with u: per-(chunk, level) partial sums of df (u_{k-1} - u_k),
+// with u: per-(block, level) partial sums of df (u_{k-1} - u_k),
 // df (u_{k+1} - u_k), df and u.  The row and column of an element advance by
-// the block's stride without a division (a 64-bit one per element made this
-// kernel issue-bound: 58 us at 256 x 256 x 128).
+// the blocks' stride without a division (a 64-bit one per element made this
+// kernel issue-bound: 58 us at 256 x 256 x 128).  The blocks of a level take
+// its rows of 256 elements in turn, so that each thread's and each block's
+// partial sum runs over the whole plane: the terms of a smooth field cancel
+// there, where sums over contiguous pieces grow large before they cancel
+// across the pieces (ddmx3 of 70 problems 10 % further from 64 bits with
+// 4096-cell pieces, 540 us a gradient of 256 x 256 x 128; in turn as near as
+// one block a 16384-cell piece, 541 us).
 template <bool GRAD>
 __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ W, double* __restrict__ df,
                                                       const double* __restrict__ dx3, const double* __restrict__ corr,
                                                       const double* __restrict__ u, int nx, int ny, int nz, long sy,
-                                                      long sz, int chunk, int nchunk, double* __restrict__ mpart)
+                                                      long sz, int nchunk, double* __restrict__ mpart)
 {
     __shared__ double red[ADJ_TPB / 32];
     const int k = blockIdx.y;
-    const int plane = nx * ny;
-    const int i0 = blockIdx.x * chunk, i1 = min(plane, i0 + chunk);
+    const int plane = nx * ny, step = nchunk * ADJ_TPB;
     const double s3 = dx3[k + 1], ck = corr[k];
-    const int dj = ADJ_TPB / nx, di = ADJ_TPB - dj * nx;
+    const int dj = step / nx, di = step - dj * nx;
     const double* const Wk = W + (long)(k + 1) * sz + sy + 1;
     const double* const uk = GRAD ? u + (long)(k + 1) * sz + sy + 1 : nullptr;
     double* const dk = df + (long)k * plane;
     const long lo = k > 0 ? -sz : 0, hi = k < nz - 1 ? sz : 0;   // the walls' terms are zero
     double sm = 0.0, sp = 0.0, sd = 0.0, su = 0.0;
-    int e = i0 + (int)threadIdx.x;
+    int e = blockIdx.x * ADJ_TPB + (int)threadIdx.x;
     int j = e / nx, i = e - j * nx;
     auto next = [&]() -> int {
         const int o = i + j * (int)sy;
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ 
         }
     };
     constexpr int Q = 4;   // elements in flight
-    for (; e + (Q - 1) * ADJ_TPB < i1; e += Q * ADJ_TPB) {
+    for (; e + (Q - 1) * step < plane; e += Q * step) {
         double w[Q], uc[Q], um[Q], up[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -205,9 +210,9 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ 
             if constexpr (GRAD) { uc[q] = uk[o]; um[q] = uk[o + lo]; up[q] = uk[o + hi]; }
         }
 #pragma unroll
-        for (int q = 0; q < Q; ++q) one(w[q], e + q * ADJ_TPB, uc[q], um[q], up[q]);
+        for (int q = 0; q < Q; ++q) one(w[q], e + q * step, uc[q], um[q], up[q]);
     }
-    for (; e < i1; e += ADJ_TPB) {
+    for (; e < plane; e += step) {
         const int o = next();
         if constexpr (GRAD) one(Wk[o], e, uk[o], uk[o + lo], uk[o + hi]);
         else one(Wk[o], e, 0.0, 0.0, 0.0);
@@ -301,11 +306,11 @@ cudaError_t launch_adj_rhs(const double* g, double* h, const double* dx3, const 
 }
 
 cudaError_t launch_adj_out(const double* W, double* df, const double* dx3, const double* corr, const double* u,
-                           const Geom& gm, long chunk, int nchunk, double* mpart, cudaStream_t st)
+                           const Geom& gm, int nchunk, double* mpart, cudaStream_t st)
 {
     auto kern = u ? k_adj_out<true> : k_adj_out<false>;
     kern<<<dim3(nchunk, gm.nz), ADJ_TPB, 0, st>>>(W, df, dx3, corr, u, gm.nx, gm.ny, gm.nz, gm.pstride_y, gm.pstride_z,
-                                                 (int)chunk, nchunk, mpart);
+                                                 nchunk, mpart);
     return cudaGetLastError();
 }
 

@@ -627,7 +627,7 @@ int adjoint_impl(ppf_plan* p, const double* g, double* df, const double* u, doub
     // computes the z coefficients am, ap used below
     int rc = solve_impl(p, df, p->adj_W, dmx1, dmx2, dmx3, dx3, st);
     if (rc != PPF_OK) return rc;
-    e = launch_adj_out(p->adj_W, df, dx3, corr, (ddx3 || ddmx3) ? u : nullptr, gm, p->adj_chunk, nch, mpart, st);
+    e = launch_adj_out(p->adj_W, df, dx3, corr, (ddx3 || ddmx3) ? u : nullptr, gm, nch, mpart, st);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint output");
     if (ddx3 || ddmx3) {
         e = launch_adj_metric(mpart, nch, gm, p->am, p->ap, dx3, dmx3, ddx3, ddmx3, wk, st);
