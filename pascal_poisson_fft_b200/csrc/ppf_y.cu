@@ -352,7 +352,7 @@ cudaError_t launch_yfwd(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
                                               skip_flag);
         };
         // several waves of blocks: more than 1024 threads for each SM
-        bool wide = false;
+        [[maybe_unused]] bool wide = false;
         if constexpr (!SH::CT && sizeof(T) == 8) {
             int sms = 0;
             err = device_sms(&sms);
@@ -399,7 +399,7 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
                                               dc_shift, skip_flag);
         };
         // several waves of blocks: more than 1024 threads for each SM
-        bool wide = false;
+        [[maybe_unused]] bool wide = false;
         if constexpr (!SH::CT && sizeof(T) == 8) {
             int sms = 0;
             err = device_sms(&sms);
