@@ -281,9 +281,16 @@ int ztab_rows(const ppf_plan* p) { return p->ykind == Y_C2C ? p->my / 2 + 1 : p-
 // -> 182, 256^3 real (134) 533 -> 538; cyclic (two tables) 96 x 96 x 200 (29)
 // 244 -> 174, 256 x 256 x 513 (303) 987 -> 1025.  Mixed, one sweep: 128^3 225 ->
 // 208; real data (an entry is three times its value) 128 x 128 x 256 (17)
-// 377 -> 367.  Mixed solves of tall columns on few cells have no transform long enough to
-// hide the table's chains (128 x 128 x 200 262 -> 274 us), unless the plane is too small to fill the chip (48 x 48
-// x 512 550 -> 297).  The problems of a batch hide their chains behind one
+// 377 -> 367.  FP32 spectra of tall columns on few cells have no transform long
+// enough to hide the table's chains, mixed (one sweep) and FP32 solve: 128 x
+// 128 x 200 213 -> 219, 110 = 110 us; 96 x 96 x 400 369 -> 371, 197 -> 204; 96
+// x 80 x 600 487 -> 494, 256 -> 277; unless the plane is too small to fill the
+// chip (48 x 48 x 512 500 -> 271, 271 -> 167; but 64 x 64 x 512 304 -> 309,
+// 172 -> 186).  The line at 160 levels and 5 M cells is a coarse one: of
+// the grids it leaves out, the widest planes would gain (160 x 160 x 192 334
+// -> 322, 174 -> 164; 144 x 144 x 240 374 -> 360, 193 -> 183), and of those
+// above it 160 x 160 x 200 stays as it is (345 -> 346, 180 -> 175) and 128 x 128 x
+// 512 loses in FP32 (473 -> 466, 234 -> 243).  The problems of a batch hide their chains behind one
 // another and would pay the tables' bytes: 64 FP64 problems 8.14 -> 8.70 ms.
 long plan_ztab(const ppf_plan* p)
 {

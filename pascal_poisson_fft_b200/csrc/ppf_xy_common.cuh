@@ -49,7 +49,7 @@ inline int pick_w(int n, int& threads)
 }
 
 // Compile-time shapes of the common lengths: W lines, NT threads (8 elements
-// a thread, 16 in the FP32 32- and 512-point tiles), radix sequence.  Other
+// a thread, 16 in the FP32 32-, 512- and 768-point tiles), radix sequence.  Other
 // lengths use the run-time engine.  The short lines' tiles are kept small (16
 // lines of 64 points, 8 FP64 or 16 FP32 lines of 128) so that small grids
 // have tiles for every SM and enough resident; FP32 tiles of 16 columns also
