@@ -47,7 +47,11 @@ struct PipeShape<double, ShapeCT<N, W, 512, RS...>> {
 // 320-thread blocks of a 320-point tile fit an SM instead of two: 320 x 320 x
 // 64 211 -> 199 us.  That build spills a few bytes, and a kernel with local
 // memory does not overlap its launch with the previous kernel: 100 x 90 x 33
-// 53 -> 59 us, so grids without several waves of blocks take the other.)
+// 53 -> 59 us, so grids without several waves of blocks take the other.  The
+// y inverse of the complex kinds takes WIDE at every size: its other build, 68
+// to 70 registers, gains on a few grids (48 x 500 x 30 57 -> 54 us) and loses
+// more on others, where a second wave follows (40 x 640 x 71 107 -> 116, 192
+// x 180 x 51 82 -> 89).)
 template <typename SH> constexpr int y_threads = SH::CT ? SH::NT : 512;
 template <typename SH, bool WIDE> constexpr int y_ctas = !SH::CT ? (WIDE ? 2 : 0) : SH::NT <= 256 ? 1024 / SH::NT : 2;
 
@@ -408,10 +412,12 @@ cudaError_t launch_yinv(int kind, const cx<T>* in, long in_pitch, cx<T>* out, lo
         }
         auto pick = [&](auto k) {
             constexpr int KIND = decltype(k)::value;
-            if constexpr (!SH::CT && sizeof(T) == 8) {
+            // (complex kinds: the 64-register build at every size)
+            constexpr bool one = !SH::CT && sizeof(T) == 8 && KIND != Y_RPAIR;
+            if constexpr (!SH::CT && sizeof(T) == 8 && !one) {
                 if (wide) { go(k_yinv<T, KIND, SH, true>); return; }
             }
-            go(k_yinv<T, KIND, SH>);
+            go(k_yinv<T, KIND, SH, one>);
         };
         if (kind == Y_C2C) {
             if constexpr (SH::CT)
