@@ -163,8 +163,10 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_rhs(const double* g, double* h,
 // partial sum runs over the whole plane: the terms of a smooth field cancel
 // there, where sums over contiguous pieces grow large before they cancel
 // across the pieces (ddmx3 of 70 problems 10 % further from 64 bits with
-// 4096-cell pieces, 540 us a gradient of 256 x 256 x 128; in turn as near as
-// one block a 16384-cell piece, 541 us).
+// 4096-cell pieces than with 16384-cell ones; in turn as near as the latter,
+// at the same 540 us a gradient of 256 x 256 x 128).  A thread's last elements
+// load together as the others do: one by one 162 x 300 x 120 takes 553 us
+// instead of 547.
 template <bool GRAD>
 __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ W, double* __restrict__ df,
                                                       const double* __restrict__ dx3, const double* __restrict__ corr,
@@ -212,10 +214,20 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_out(const double* __restrict__ 
 #pragma unroll
         for (int q = 0; q < Q; ++q) one(w[q], e + q * step, uc[q], um[q], up[q]);
     }
-    for (; e < plane; e += step) {
-        const int o = next();
-        if constexpr (GRAD) one(Wk[o], e, uk[o], uk[o + lo], uk[o + hi]);
-        else one(Wk[o], e, 0.0, 0.0, 0.0);
+    if (e < plane) {
+        // the last elements, their loads in flight as well
+        double w[Q - 1], uc[Q - 1], um[Q - 1], up[Q - 1];
+#pragma unroll
+        for (int q = 0; q < Q - 1; ++q) {
+            const int o = next();
+            if (e + q * step < plane) {
+                w[q] = Wk[o];
+                if constexpr (GRAD) { uc[q] = uk[o]; um[q] = uk[o + lo]; up[q] = uk[o + hi]; }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q - 1; ++q)
+            if (e + q * step < plane) one(w[q], e + q * step, uc[q], um[q], up[q]);
     }
     if constexpr (GRAD) {
         sm = block_sum(sm, red);
